@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB)
     }
     const ParkOut out{park + G.park_off, G.park_cap, counts + s_seg};
     if (run_or_park<EXTRAS, K>(P, S, PL, active, G.stage_cap, out) || !active) return;
-    const V3 c = path_finish<1, false, K>(P, S, B);
+    const V3 c = path_finish<1, false, K, EXTRAS>(P, S, B);
     float *xyz = G.xyz;
     xyz[3 * t + 0] = c.x;
     xyz[3 * t + 1] = c.y;

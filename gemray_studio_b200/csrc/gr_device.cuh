@@ -71,13 +71,16 @@ struct SceneConst {
     float d_beta_alpha;
     uint32_t has_beta, n_b_bands;
     float b_bands[GR_MAX_BANDS][3];
+    uint32_t sane;  // every input finite and every index in (1.01, 8) (sane_scene)
 };
 
-// Scenes that need the extension instantiation of the transport kernels (frosted
-// facets, volume scattering, biaxial materials); every other scene runs the default
-// instantiation, which contains none of that code.
+// Scenes that need the extension instantiation of the transport kernels: frosted facets,
+// volume scattering, biaxial materials -- and scenes whose arithmetic may leave the finite
+// range, since the extension instantiation alone computes every term and every channel
+// (live_only, gr_trace.cuh).  Every other scene runs the default instantiation, which
+// contains none of that code.
 __host__ __device__ inline bool needs_extras(const SceneConst &S) {
-    return S.any_frosted || S.sigma_s > 0.0f || S.biaxial;
+    return S.any_frosted || S.sigma_s > 0.0f || S.biaxial || !S.sane;
 }
 
 struct SceneBuffers {

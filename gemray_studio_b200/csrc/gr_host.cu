@@ -193,6 +193,73 @@ gr_status validate_scene(const gr_scene *sc) {
 }
 
 
+// Whether the transport of this scene stays finite: every number it reads is finite and
+// bounded, and the refractive indices over [380, 780] nm lie within (1.01, 8), so that no
+// Fresnel denominator vanishes.  The dispersion terms are monotonic in the wavelength
+// where they have no pole, so their values at the two ends bound them.  (A lat-long map is
+// checked texel by texel where it is read.)
+static bool sane_scene(const gr_scene *sc, const SceneConst &S) {
+    bool ok = true;
+    auto within = [&ok](float v, float most) { ok = ok && fabsf(v) <= most; };  // false for NaN
+    auto within_n = [&](const float *v, size_t n, float most) { for (size_t i = 0; i < n; ++i) within(v[i], most); };
+    within_n(S.cam_o, 3, 1e6f);
+    within_n(S.cam_f, 3, 1e6f);
+    within_n(S.cam_r, 3, 1e6f);
+    within_n(S.cam_u, 3, 1e6f);
+    within(S.fov_tan, 1e6f);
+    if (sc->planes) within_n(&sc->planes[0].normal[0], (size_t)sc->n_planes * 4, 1e6f);
+    within_n(S.c_axis, 3, 1e6f);
+    within(S.path_scale, 1e6f);
+    within(S.edge_radius, 1e6f);
+    within_n(S.uni_rgb, 3, 1e15f);
+    within(S.temp_k, 1e15f);
+    within(S.spot_mult, 1e9f);
+    within(S.exposure, 1e9f);
+    for (const auto *bands : {S.o_bands, S.e_bands}) {
+        const uint32_t n = bands == S.o_bands ? S.n_o_bands : S.n_e_bands;
+        for (uint32_t i = 0; i < n; ++i) {
+            within_n(bands[i], 3, 1e6f);
+            ok = ok && fabsf(bands[i][1]) >= 1e-3f;
+        }
+    }
+    for (uint32_t i = 0; i < S.ext_n; ++i) {
+        within(sc->material_ext->alpha_o_table[i], 1e6f);
+        within(sc->material_ext->alpha_e_table[i], 1e6f);
+    }
+    if (S.ext_n) ok = ok && S.ext_step >= 1e-6f && fabsf(S.ext_first) <= 1e6f;
+    // bounds of n (Cauchy) or n^2 (Sellmeier) from each term's values at both ends
+    const float ends[2] = {0.380f * 0.380f, 0.780f * 0.780f};
+    auto add_term = [](float a, float b, float &lo, float &hi) { lo += fminf(a, b); hi += fmaxf(a, b); };
+    auto cauchy = [&](const float *c, float &lo, float &hi) {
+        lo = hi = c[0];
+        add_term(c[1] / ends[0], c[1] / ends[1], lo, hi);
+        add_term(c[2] / (ends[0] * ends[0]), c[2] / (ends[1] * ends[1]), lo, hi);
+    };
+    float lo, hi;
+    if (S.disp_model == GR_DISP_CAUCHY) {
+        cauchy(S.disp_a, lo, hi);
+    } else {
+        lo = hi = 1.0f;
+        const int terms = S.disp_model == GR_DISP_SELLMEIER1 ? 1 : 3;
+        for (int i = 0; i < terms; ++i) {
+            const float a = S.disp_a[i], b = S.disp_b[i];
+            if (a == 0.0f && fabsf(b) <= 1e6f && (b < 0.14f || b > 0.62f)) continue;
+            ok = ok && fabsf(a) <= 1e6f && (b <= 0.14f || b >= 0.62f) && fabsf(b) <= 1e6f;  // no pole in the range
+            add_term(a * ends[0] / (ends[0] - b), a * ends[1] / (ends[1] - b), lo, hi);
+        }
+        lo = sqrtf(fmaxf(lo, 0.0f));
+        hi = sqrtf(fmaxf(hi, 0.0f));
+    }
+    ok = ok && lo > 1.01f && hi < 8.0f;
+    if (S.has_cauchy_e) {
+        cauchy(S.cauchy_e, lo, hi);
+    } else {
+        lo += S.bire;
+        hi += S.bire;
+    }
+    return ok && lo > 1.01f && hi < 8.0f;
+}
+
 void encode_scene(const gr_scene *sc, SceneConst &S) {
     std::memset(&S, 0, sizeof(S));
     for (int i = 0; i < 3; ++i) {
@@ -277,6 +344,7 @@ void encode_scene(const gr_scene *sc, SceneConst &S) {
     S.map_w = sc->env.latlong_w;
     S.map_h = sc->env.latlong_h;
     S.flags = sc->flags;
+    S.sane = sane_scene(sc, S) ? 1u : 0u;
 }
 
 }  // namespace grh

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, GR_TRACE_MIN_BLOCKS) k_trace_st
         else if (ev == EV_REFRACT) step_refract<1, NoCounters, EXTRAS>(P, S, E, nc);
     }
     float4 s4;
-    const V3 c = path_finish<1, true>(P, S, B, &s4);
+    const V3 c = path_finish<1, true, K_ANY, EXTRAS>(P, S, B, &s4);
     xyz[3 * t + 0] = c.x;
     xyz[3 * t + 1] = c.y;
     xyz[3 * t + 2] = c.z;

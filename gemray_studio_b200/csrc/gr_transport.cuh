@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_stage1(SceneConst S
         path_init<1, EXTRAS, K>(P, S, B, pixel, sample, (uint32_t)t);
     }
     if (run_or_park<EXTRAS, K>(P, S, PL, active, bounce_cap, out) || !active) return;
-    const V3 c = path_finish<1, false, K>(P, S, B);
+    const V3 c = path_finish<1, false, K, EXTRAS>(P, S, B);
     xyz[3 * t + 0] = c.x;
     xyz[3 * t + 1] = c.y;
     xyz[3 * t + 2] = c.z;
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_stage2(
     Path P;
     if (active) P = park_in[i];
     if (run_or_park<EXTRAS, K>(P, S, PL, active, bounce_cap, out) || !active) return;
-    const V3 c = path_finish<1, false, K>(P, S, B);
+    const V3 c = path_finish<1, false, K, EXTRAS>(P, S, B);
     const uint64_t t = p_tuple(P);
     xyz[3 * t + 0] = c.x;
     xyz[3 * t + 1] = c.y;

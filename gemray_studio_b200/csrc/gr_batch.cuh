@@ -80,10 +80,10 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB)
     if (active) {
         uint32_t pixel, sample;
         tuple_coords(R, t, pixel, sample);
-        path_init<1, EXTRAS, K>(P, S, B, pixel, sample, (uint32_t)t);
+        path_init<K>(P, S, pixel, sample, (uint32_t)t);
     }
     const ParkOut out{park + G.park_off, G.park_cap, counts + s_seg};
-    if (run_or_park<EXTRAS, K>(P, S, PL, active, G.stage_cap, out) || !active) return;
+    if (run_or_park<EXTRAS, K>(P, S, B, PL, active, G.stage_cap, out) || !active) return;
     const V3 c = path_finish<1, false, K, EXTRAS>(P, S, B);
     float *xyz = G.xyz;
     xyz[3 * t + 0] = c.x;

@@ -171,7 +171,10 @@ __device__ __forceinline__ float exp_poly(float x) {
     const float C2 = -2.1219444e-4f;
     if (x < -87.33654f) x = -87.33654f;
     if (x > 88.02875f) x = 88.02875f;
-    float n = floorf(fmaf(x, LOG2E, 0.5f));
+    // floor(v), |v| < 2^22: the sum rounded down to a spacing of 1 keeps it in the low
+    // mantissa bits, as a float by subtracting again and as the exponent by a shift
+    const float biased = __fadd_rd(fmaf(x, LOG2E, 0.5f), 12582912.0f);  // 1.5 * 2^23
+    const float n = biased - 12582912.0f;
     x = fmaf(n, -C1, x);
     x = fmaf(n, -C2, x);
     float z = x * x;
@@ -182,7 +185,16 @@ __device__ __forceinline__ float exp_poly(float x) {
     p = fmaf(p, x, 1.6666665e-1f);
     p = fmaf(p, x, 5.0000003e-1f);
     p = fmaf(p, z, x) + 1.0f;
-    return p * __uint_as_float((uint32_t)(((int)n + 127) << 23));
+    return p * __uint_as_float((__float_as_uint(biased) + 127u) << 23);
+}
+
+// a / c for a constant c whose correctly rounded reciprocal is rc: the quotient's estimate
+// a * rc corrected once by its exact remainder (Markstein, IBM J. Res. Dev. 34, 1990).
+// Without a range check: exact for the operands used here, which tests/test_exact_division.py
+// shows for every wavelength in [380, 780] nm and every constant.
+__device__ __forceinline__ float div_const(float a, float c, float rc) {
+    const float q = a * rc;
+    return fmaf(fmaf(-c, q, a), rc, q);
 }
 
 // ---------------------------------------------------------------------------------
@@ -198,13 +210,27 @@ __device__ __forceinline__ uint32_t hash_u32(uint32_t x) {  // sampling.rs:45-51
 __device__ __forceinline__ float ld_base2(uint32_t n) {  // sampling.rs:139-147
     return (float)__brev(n) / 4294967296.0f;
 }
+// The digit weights of radical_inverse<BASE>: 1/BASE divided by BASE again and again, each
+// quotient rounded to f32 (21 base-3 or 14 base-5 digits hold every u32).
+template <uint32_t BASE> struct RadicalWeights {
+    float w[21];
+    constexpr RadicalWeights() : w{} {
+        float v = 1.0f / (float)BASE;
+        for (int i = 0; i < 21; ++i) {
+            w[i] = v;
+            v = v / (float)BASE;
+        }
+    }
+};
+static __constant__ constexpr RadicalWeights<3> kRadical3{};
+static __constant__ constexpr RadicalWeights<5> kRadical5{};
 template <uint32_t BASE> __device__ __forceinline__ float radical_inverse(uint32_t n) {  // sampling.rs:170-181
+    static_assert(BASE == 3 || BASE == 5, "weights tabulated for the sampler's bases");
+    const float *w = BASE == 3 ? kRadical3.w : kRadical5.w;
     float val = 0.0f;
-    float inv_base = 1.0f / (float)BASE;
     while (n > 0) {
         uint32_t digit = n % BASE;
-        val = fmaf((float)digit, inv_base, val);
-        inv_base = inv_base / (float)BASE;
+        val = fmaf((float)digit, *w++, val);
         n /= BASE;
     }
     return val;
@@ -254,7 +280,8 @@ __device__ __forceinline__ Draws sample_draws(uint32_t pixel, uint32_t sample) {
 __device__ __forceinline__ float lambda_k(float hero, int k) {
     float lh = fmaf(hero, 400.0f, 380.0f);
     float off = fmaf((float)k, 50.0f, lh - 380.0f);
-    return 380.0f + rem_euclid(off, 400.0f);
+    // off rem_euclid 400 for off in [0, 800): the difference is exact there, as fmod is
+    return 380.0f + (off >= 400.0f ? off - 400.0f : off);
 }
 // dispersion.rs:12-37
 __device__ __forceinline__ float dispersion(const SceneConst &S, float lambda_nm) {
@@ -604,29 +631,58 @@ __device__ __forceinline__ float blackbody(const SceneConst &S, float lambda_nm)
     float ratio = S.denom560 / denom;
     return clampf(powi<5>(560.0f / lambda_nm) * ratio, 0.01f, 20.0f);
 }
-// environment.rs:280-321
-__device__ __forceinline__ float studio_radiance(const SceneConst &S, V3 dn, float lambda_nm) {
-    float spec = blackbody(S, lambda_nm);
-    float bg = fmaxf(fmaf(0.012f, fmaf(dn.y, 0.5f, 0.5f), 0.015f), 0.005f) * S.exposure;
-    float rad = bg * spec;
+// environment.rs:280-321.  The lights' weights depend on the direction alone, so they are
+// formed once per path (StudioTerms) and each wavelength adds them in the reference's
+// order: background, key, fill, then the ring lights that shine (at most the few within
+// 16 degrees of the direction, of 16).
+struct StudioTerms {
+    float bg, key, fill;
+    uint32_t lights;  // bit 0: key, bit 1: fill, bits 8..: number of ring lights
+    float ring[16];
+};
+__device__ __forceinline__ void studio_terms(const SceneConst &S, V3 dn, StudioTerms &T) {
+    T.bg = fmaxf(fmaf(0.012f, fmaf(dn.y, 0.5f, 0.5f), 0.015f), 0.005f) * S.exposure;
+    T.key = T.fill = 0.0f;
+    uint32_t lights = 0, n = 0;
     float key_dot = fmaxf(dot(dn, ld3(S.key)), 0.0f);
-    if (key_dot > 0.0f) rad = fmaf(powi<28>(key_dot) * 12.0f * S.spot_mult * S.exposure, spec, rad);
+    if (key_dot > 0.0f) {
+        T.key = powi<28>(key_dot) * 12.0f * S.spot_mult * S.exposure;
+        lights |= 1u;
+    }
     float fill_dot = fmaxf(dot(dn, ld3(S.fill)), 0.0f);
-    if (fill_dot > 0.0f) rad = fmaf(powi<18>(fill_dot) * 4.5f * S.exposure, spec, rad);
-#pragma unroll 4
+    if (fill_dot > 0.0f) {
+        T.fill = powi<18>(fill_dot) * 4.5f * S.exposure;
+        lights |= 2u;
+    }
+#pragma unroll 1
     for (int i = 0; i < 16; ++i) {
         float ring_dot = fmaxf(dot(dn, ld3(S.ring[i])), 0.0f);
         if (ring_dot > 0.96f) {
             float spark = (ring_dot - 0.96f) / 0.04f;
-            rad = fmaf(powi<6>(spark) * 22.0f * S.spot_mult * S.exposure, spec, rad);
+            T.ring[n++] = powi<6>(spark) * 22.0f * S.spot_mult * S.exposure;
         }
     }
+    T.lights = lights | (n << 8);
+}
+__device__ __forceinline__ float studio_spectrum(const SceneConst &S, const StudioTerms &T, float lambda_nm) {
+    float spec = blackbody(S, lambda_nm);
+    float rad = T.bg * spec;
+    if (T.lights & 1u) rad = fmaf(T.key, spec, rad);
+    if (T.lights & 2u) rad = fmaf(T.fill, spec, rad);
+    const uint32_t n = T.lights >> 8;
+#pragma unroll 1
+    for (uint32_t i = 0; i < n; ++i) rad = fmaf(T.ring[i], spec, rad);
     return rad;
+}
+__device__ __forceinline__ float studio_radiance(const SceneConst &S, V3 dn, float lambda_nm) {
+    StudioTerms T;
+    studio_terms(S, dn, T);
+    return studio_spectrum(S, T, lambda_nm);
 }
 // env_map_spectrum.rs asymmetric_gaussian / rgb_to_spectral_radiance
 __device__ __forceinline__ float asym_gauss(float x, float mu, float slo, float shi) {
-    float sigma = x < mu ? slo : shi;
-    float t = (x - mu) / sigma;
+    const bool lo = x < mu;
+    const float t = div_const(x - mu, lo ? slo : shi, lo ? 1.0f / slo : 1.0f / shi);
     return m_exp(-0.5f * t * t);
 }
 __device__ __forceinline__ float rgb_to_spectral(float r, float g, float b, float lambda_nm) {
@@ -670,8 +726,8 @@ __device__ __forceinline__ void latlong_rgb(const SceneConst &S, const float *__
 // a14. CIE 1931 via the reference polynomial exp (color/cie1931.rs:78-98)
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ float lobe(float l, float mu, float slo, float shi) {
-    float sigma = l < mu ? slo : shi;
-    float t = (l - mu) / sigma;
+    const bool lo = l < mu;
+    const float t = div_const(l - mu, lo ? slo : shi, lo ? 1.0f / slo : 1.0f / shi);
     return exp_poly(-0.5f * t * t);
 }
 __device__ __forceinline__ V3 cmf(float l) {

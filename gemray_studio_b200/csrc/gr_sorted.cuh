@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(SORT_THREADS, GR_SORT_MIN_BLOCKS) k_trace_sort
             if (claim && t < R.n_tuples) {
                 uint32_t pixel, sample;
                 tuple_coords(R, t, pixel, sample);
-                path_init<1, false, K>(P, S, B, pixel, sample, (uint32_t)t);
+                path_init<K>(P, S, pixel, sample, (uint32_t)t);
                 sh.state[slot] = SLOT_LIVE;
             } else {
                 sh.state[slot] = SLOT_EMPTY;
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(SORT_THREADS, GR_SORT_MIN_BLOCKS) k_trace_sort
         if (n_live == 0) break;  // block-uniform: nothing live and nothing left to start
         if (tid < n_live) {
             const uint32_t slot = sh.list_a[tid];
-            sh.ev[slot] = (uint8_t)step_hit<1, NoCounters, false, false, K>(slot_path(slots, slot), S, PL,
+            sh.ev[slot] = (uint8_t)step_hit<1, NoCounters, false, false, K>(slot_path(slots, slot), S, B, PL,
                                                                             slot_event(slots, slot), nc);
         }
         __syncthreads();

@@ -33,11 +33,11 @@ __global__ void __launch_bounds__(TRACE_THREADS, GR_TRACE_MIN_BLOCKS) k_trace_st
     uint32_t pixel, sample;
     tuple_coords(R, t, pixel, sample);
     Path P;
-    path_init<1, EXTRAS>(P, S, B, pixel, sample, (uint32_t)t);
+    path_init(P, S, pixel, sample, (uint32_t)t);
     NoCounters nc;
     while (state_bits(P) & F_ALIVE) {
         Event E;
-        const uint32_t ev = step_hit<1, NoCounters, false, EXTRAS>(P, S, PL, E, nc);
+        const uint32_t ev = step_hit<1, NoCounters, false, EXTRAS>(P, S, B, PL, E, nc);
         if (ev == EV_REFLECT) step_reflect<1, NoCounters, EXTRAS>(P, S, E, nc);
         else if (ev == EV_REFRACT) step_refract<1, NoCounters, EXTRAS>(P, S, E, nc);
     }

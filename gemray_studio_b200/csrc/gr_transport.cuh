@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_plain(SceneConst S,
         uint32_t pixel, sample;
         tuple_coords(R, t, pixel, sample);
         Path P;
-        path_init<1, EXTRAS, K>(P, S, B, pixel, sample, (uint32_t)t);
+        path_init<K>(P, S, pixel, sample, (uint32_t)t);
         tally(ct, C_PATHS);
         V3 c = trace_path<CT, RESOLVE, EXTRAS, K>(P, S, B, PL, ct);
         xyz[3 * t + 0] = c.x;
@@ -63,9 +63,9 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_stage1(SceneConst S
     if (active) {
         uint32_t pixel, sample;
         tuple_coords(R, t, pixel, sample);
-        path_init<1, EXTRAS, K>(P, S, B, pixel, sample, (uint32_t)t);
+        path_init<K>(P, S, pixel, sample, (uint32_t)t);
     }
-    if (run_or_park<EXTRAS, K>(P, S, PL, active, bounce_cap, out) || !active) return;
+    if (run_or_park<EXTRAS, K>(P, S, B, PL, active, bounce_cap, out) || !active) return;
     const V3 c = path_finish<1, false, K, EXTRAS>(P, S, B);
     xyz[3 * t + 0] = c.x;
     xyz[3 * t + 1] = c.y;
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_stage2(
     const bool active = i < n;
     Path P;
     if (active) P = park_in[i];
-    if (run_or_park<EXTRAS, K>(P, S, PL, active, bounce_cap, out) || !active) return;
+    if (run_or_park<EXTRAS, K>(P, S, B, PL, active, bounce_cap, out) || !active) return;
     const V3 c = path_finish<1, false, K, EXTRAS>(P, S, B);
     const uint64_t t = p_tuple(P);
     xyz[3 * t + 0] = c.x;

@@ -40,10 +40,10 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_trace_events(SceneConst S, Sc
     uint32_t pixel, sample;
     tuple_coords(R, t, pixel, sample);
     Path P;
-    path_init<1, EXTRAS>(P, S, B, pixel, sample, (uint32_t)t);
+    path_init(P, S, pixel, sample, (uint32_t)t);
     while (state_bits(P) & F_ALIVE) {
         Event E;
-        const uint32_t ev = step_hit<1, EventRec, false, EXTRAS>(P, S, PL, E, r);
+        const uint32_t ev = step_hit<1, EventRec, false, EXTRAS>(P, S, B, PL, E, r);
         if (ev == EV_REFLECT) step_reflect<1, EventRec, EXTRAS>(P, S, E, r);
         else if (ev == EV_REFRACT) step_refract<1, EventRec, EXTRAS>(P, S, E, r);
     }

@@ -360,6 +360,21 @@ __device__ __forceinline__ Stokes apply_tir(const Stokes &s, float cd, float sd)
     o.v = ((0.0f * s.i + 0.0f * s.q) + (-sd) * s.u) + cd * s.v;
     return o;
 }
+// The same three for finite Stokes vectors with I >= +0 (the default kernels: SceneConst::sane
+// and physical intensities): there a zero entry contributes +-0, which changes no sum but
+// the sign of one that is zero.  `+ 0.0f` keeps that sign, which an atan2 may read (the
+// E-field direction of an absorbing stone); CLEAR stones have no such reader, and zeros of
+// either sign give them the same intensities.
+template <bool CLEAR> __device__ __forceinline__ float zero_sign(float v) { return CLEAR ? v : v + 0.0f; }
+template <bool CLEAR> __device__ __forceinline__ Stokes rotate_finite(const Stokes &s, float c2, float s2) {
+    return Stokes{s.i, zero_sign<CLEAR>(c2 * s.q + s2 * s.u), zero_sign<CLEAR>((-s2) * s.q + c2 * s.u), zero_sign<CLEAR>(s.v)};
+}
+template <bool CLEAR> __device__ __forceinline__ Stokes fresnel_finite(const Stokes &s, float a, float b, float c) {
+    return Stokes{a * s.i + b * s.q, zero_sign<CLEAR>(b * s.i + a * s.q), zero_sign<CLEAR>(c * s.u), zero_sign<CLEAR>(c * s.v)};
+}
+template <bool CLEAR> __device__ __forceinline__ Stokes tir_finite(const Stokes &s, float cd, float sd) {
+    return Stokes{s.i, zero_sign<CLEAR>(s.q), zero_sign<CLEAR>(cd * s.u + sd * s.v), zero_sign<CLEAR>((-sd) * s.u + cd * s.v)};
+}
 // Rust f32::midpoint on x86_64 == correctly rounded (a+b)/2 == (a+b)*0.5 in f32 for
 // every non-subnormal sum.
 __device__ __forceinline__ float midpoint(float a, float b) { return (a + b) * 0.5f; }

@@ -783,7 +783,9 @@ __device__ __forceinline__ uint32_t step_hit(Path &P, const SceneConst &S, const
         float2 sc = m_sincos(2.0f * psi);
         each_channel<live_only<CT, X>, rot_unroll(K)>(live, [&](int k) {
             float4 s = P.st[k];
-            Stokes r = apply_rotation(Stokes{s.x, s.y, s.z, s.w}, sc.y, sc.x);
+            const Stokes in{s.x, s.y, s.z, s.w};
+            const Stokes r = live_only<CT, X> ? rotate_finite<(K & K_CLEAR) != 0>(in, sc.y, sc.x)
+                                              : apply_rotation(in, sc.y, sc.x);
             P.st[k] = make_float4(r.i, r.q, r.u, r.v);
         });
         tally(ct, C_ROTATIONS);
@@ -837,7 +839,7 @@ __device__ __forceinline__ uint32_t step_hit(Path &P, const SceneConst &S, const
     const float n_med0 = n_med<K>(P, E, 0);
     const float n1 = inside ? n_med0 : 1.0f;
     const float n2 = inside ? 1.0f : n_med0;
-    const float eta0 = n1 / n2;
+    const float eta0 = inside ? n_med0 : 1.0f / n_med0;
     const float sin2_t = eta0 * eta0 * one_m_c2;
     E.hp_cos = make_float4(hp.x, hp.y, hp.z, cos_i);
 
@@ -979,24 +981,25 @@ __device__ __forceinline__ void step_reflect(Path &P, const SceneConst &S, const
     // A TIR event applies each channel's matrix unscaled: the reflect branch's
     // `.scale(1 / r_unpol)` with factor 1.0 (x * 1.0f == x exactly).
     const float inv = hero_tir ? 1.0f : 1.0f / E.n_ru.w;
+    constexpr bool FIN = live_only<CT, X>, CLEAR = (K & K_CLEAR) != 0;
     each_channel<live_only<CT, X>, U>(live_channels<CT, X>(bits), [&](int k) {
         const float nm = n_med<K>(P, E, k);
         const float n1k = inside ? nm : 1.0f, n2k = inside ? 1.0f : nm;
-        const float etak = n1k / n2k;
+        const float etak = inside ? nm : 1.0f / nm;  // n1k / n2k: one of them is 1
         const float s2k = etak * etak * one_m_c2;
         float4 s4 = P.st[k];
         Stokes s{s4.x, s4.y, s4.z, s4.w};
         if (s2k > 1.0f) {
             tally(ct, C_CH_TIR);
             float2 sc = m_sincos(tir_phase_delta(n1k, cos_i, sin_i));
-            s = scale(apply_tir(s, sc.y, sc.x), inv);
+            s = scale(FIN ? tir_finite<CLEAR>(s, sc.y, sc.x) : apply_tir(s, sc.y, sc.x), inv);
         } else {
             float ctk = sqrtf(fmaxf(1.0f - s2k, 0.0f));
             float rsk, rpk, a, b, c;
             fresnel_rs_rp(n1k, n2k, cos_i, ctk, rsk, rpk);
             arr(P.pdf4, k) = arr(P.pdf4, k) * r_unpol(rsk, rpk);
             fresnel_reflection_abc(rsk, rpk, a, b, c);
-            s = scale(apply_fresnel(s, a, b, c), inv);
+            s = scale(FIN ? fresnel_finite<CLEAR>(s, a, b, c) : apply_fresnel(s, a, b, c), inv);
         }
         P.st[k] = make_float4(s.i, s.q, s.u, s.v);
     });
@@ -1038,7 +1041,7 @@ __device__ __forceinline__ void step_refract(Path &P, const SceneConst &S, const
     const bool ordinary_entry = entering_aniso && !use_e && !biax_entry;
     const bool extra_entry = entering_aniso && use_e && !biax_entry;
     const float n2_dir = ordinary_entry ? n_o_hero : n2;
-    const float eta_dir = n1 / n2_dir;
+    const float eta_dir = inside ? n1 : 1.0f / n2_dir;
     const float s2d = fminf(eta_dir * eta_dir * one_m_c2, 1.0f);
     const float ctd = sqrtf(fmaxf(1.0f - s2d, 0.0f));
     const V3 refr = normalize(add(smul(eta_dir, kk), smul(fmaf(eta_dir, cos_i, -ctd), normal)));
@@ -1049,11 +1052,12 @@ __device__ __forceinline__ void step_refract(Path &P, const SceneConst &S, const
     const float tinv = 1.0f / (1.0f - ru);
     const float TOL = 1.0f - 1e-6f;
     uint32_t ended = 0u;  // channels terminated here
+    constexpr bool FIN = live_only<CT, X>, CLEAR = (K & K_CLEAR) != 0;
     each_channel<live_only<CT, X>, U>(live_channels<CT, X>(bits), [&](int k) {
         const float n_o_k = arr(P.n_o4, k);
         const float n1k = inside ? n_med<K>(P, E, k) : 1.0f;
         const float n2k = ordinary_entry ? n_o_k : (inside ? 1.0f : n_med<K>(P, E, k));
-        const float ratio = n1k / n2k;
+        const float ratio = inside ? n1k : 1.0f / n2k;  // n1k / n2k: one of them is 1
         const float s2k = (ratio * ratio) * one_m_c2;
         float4 s4 = P.st[k];
         Stokes s{s4.x, s4.y, s4.z, s4.w};
@@ -1072,7 +1076,7 @@ __device__ __forceinline__ void step_refract(Path &P, const SceneConst &S, const
             float tp = (2.0f * n1k * cos_i) / fmaf(n1k, ctk, n2k * cos_i);
             float a, b, c;
             fresnel_transmission_abc(n1k, n2k, cos_i, ctk, ts, tp, a, b, c);
-            s = scale(apply_fresnel(s, a, b, c), tinv);
+            s = scale(FIN ? fresnel_finite<CLEAR>(s, a, b, c) : apply_fresnel(s, a, b, c), tinv);
             float rsk, rpk;
             fresnel_rs_rp(n1k, n2k, cos_i, ctk, rsk, rpk);
             arr(P.pdf4, k) = arr(P.pdf4, k) * (1.0f - r_unpol(rsk, rpk));

@@ -52,16 +52,17 @@ __device__ __forceinline__ void load_slot(SceneSlot &dst_slot, const SceneSlot *
     for (uint32_t i = threadIdx.x; i < sizeof(SceneSlot) / 4; i += blockDim.x) dst[i] = src[i];
 }
 
-// Stage 1 of a batched launch (the staged scheme of the single-scene kernels): paths
-// run up to their segment's stage cap; survivors are parked in their segment's park region
-// (`park`, slot counters `counts` per segment of the launch) for k_trace_batch_cont.
+// Stage 1 of a batched launch (the pooled scheme of the single-scene kernels): a block runs
+// its pool over one segment's run of `chunk` tuples; once they are all started, paths past
+// the segment's stage cap are parked in its park region (`park`, slot counters `counts` per
+// segment of the launch) for k_trace_batch_cont.
 // EXTRAS: the variant for launches holding a scene with frosted facets, scattering or
 // a biaxial material.  K: the scene class every segment of the launch belongs to
 // (gr_trace.cuh K_*; K_ANY: checked at run time), MB: resident blocks per SM.
 template <bool EXTRAS, int K = K_ANY, int MB = GR_TRACE_MIN_BLOCKS>
-__global__ void __launch_bounds__(TRACE_THREADS, MB)
+__global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, pool_threads<EXTRAS, K>()))
     k_trace_batch(const SceneSlot *__restrict__ slots, const BatchSegment *__restrict__ segs, uint32_t n_segs,
-                  Path *__restrict__ park, unsigned int *__restrict__ counts) {
+                  uint32_t chunk, Path *__restrict__ park, unsigned int *__restrict__ counts) {
     __shared__ SceneSlot s_slot;
     __shared__ uint32_t s_seg;
     extern __shared__ float4 s_planes[];
@@ -74,27 +75,24 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB)
     const SceneBuffers &B = s_slot.B;
     const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
     const LaunchRange R = G.R;
-    const uint64_t t = (uint64_t)(blockIdx.x - G.block_begin) * blockDim.x + threadIdx.x;
-    const bool active = t < R.n_tuples;
-    Path P;
-    if (active) {
-        uint32_t pixel, sample;
-        tuple_coords(R, t, pixel, sample);
-        path_init<K>(P, S, pixel, sample, (uint32_t)t);
-    }
-    const ParkOut out{park + G.park_off, G.park_cap, counts + s_seg};
-    if (run_or_park<EXTRAS, K>(P, S, B, PL, active, G.stage_cap, out) || !active) return;
-    const V3 c = path_finish<1, false, K, EXTRAS>(P, S, B);
+    const uint64_t first = (uint64_t)(blockIdx.x - G.block_begin) * chunk;
     float *xyz = G.xyz;
-    xyz[3 * t + 0] = c.x;
-    xyz[3 * t + 1] = c.y;
-    xyz[3 * t + 2] = c.z;
+    Path P;
+    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K>(
+        P, S, B, PL, PoolRange{first, min(first + chunk, R.n_tuples)}, G.stage_cap,
+        ParkOut{park + G.park_off, G.park_cap, counts + s_seg},
+        [&](Path &q, uint64_t t) {
+            uint32_t pixel, sample;
+            tuple_coords(R, t, pixel, sample);
+            path_init<K>(q, S, pixel, sample, (uint32_t)t);
+        },
+        [&](const Path &q) { store_sample(xyz, q, path_finish<1, false, K, EXTRAS>(q, S, B)); });
 }
 
-// Stage 2: each block resumes up to 128 parked paths of one segment (its scene in
-// shared memory, as in stage 1) and runs them to their end.
+// Stage 2: each block resumes up to a block's worth of one segment's parked paths (its scene
+// in shared memory, as in stage 1) and runs them to their end.
 template <bool EXTRAS, int K = K_ANY, int MB = GR_TRACE_MIN_BLOCKS>
-__global__ void __launch_bounds__(TRACE_THREADS, MB)
+__global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, pool_threads<EXTRAS, K>()))
     k_trace_batch_cont(const SceneSlot *__restrict__ slots, const BatchSegment *__restrict__ segs, uint32_t n_segs,
                        const Path *__restrict__ park, const unsigned int *__restrict__ counts) {
     __shared__ SceneSlot s_slot;
@@ -111,26 +109,22 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB)
     const SceneConst &S = s_slot.S;
     const SceneBuffers &B = s_slot.B;
     const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
-    const uint64_t i = j0 + threadIdx.x;
-    if (i >= n) return;
-    Path P = park[G.park_off + i];
-    NoCounters nc;
-    const V3 c = trace_path<NoCounters, false, EXTRAS, K>(P, S, B, PL, nc);
-    const uint64_t t = p_tuple(P);
+    const Path *from = park + G.park_off;
     float *xyz = G.xyz;
-    xyz[3 * t + 0] = c.x;
-    xyz[3 * t + 1] = c.y;
-    xyz[3 * t + 2] = c.z;
+    Path P;
+    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K>(
+        P, S, B, PL, PoolRange{j0, min(j0 + blockDim.x, (uint64_t)n)}, 0xFFFFFFFFu, ParkOut{nullptr, 0, nullptr},
+        [&](Path &q, uint64_t i) { copy_record<record_rows<EXTRAS, K>()>(q, from[i]); },
+        [&](const Path &q) { store_sample(xyz, q, path_finish<1, false, K, EXTRAS>(q, S, B)); });
 }
 
 // One batched launch's two trace grids for scene class K at MB blocks per SM.
 template <bool EXTRAS, int K, int MB>
-void launch_batch_grids(const SceneSlot *slots, const BatchSegment *segs, uint32_t n_segs, Path *park,
+void launch_batch_grids(const SceneSlot *slots, const BatchSegment *segs, uint32_t n_segs, uint32_t chunk, Path *park,
                         unsigned int *counts, uint64_t blocks, uint64_t park_blocks, size_t smem, cudaStream_t s) {
-    k_trace_batch<EXTRAS, K, MB><<<(unsigned)blocks, TRACE_THREADS, smem, s>>>(slots, segs, n_segs, park, counts);
-    k_trace_batch_cont<EXTRAS, K, MB><<<(unsigned)park_blocks, TRACE_THREADS, smem, s>>>(slots, segs, n_segs, park,
-                                                                                        counts);
+    constexpr int T = pool_threads<EXTRAS, K>();
+    k_trace_batch<EXTRAS, K, MB><<<(unsigned)blocks, T, smem, s>>>(slots, segs, n_segs, chunk, park, counts);
+    k_trace_batch_cont<EXTRAS, K, MB><<<(unsigned)park_blocks, T, smem, s>>>(slots, segs, n_segs, park, counts);
 }
-
 
 }  // namespace grd

@@ -5,26 +5,23 @@
 #include "gr_batch.cuh"
 #include "gr_ctx.h"
 
-// Resident blocks per SM of the class-specialised batched grids.  Measured on B200
-// with the c4 stones (batched path-samples/s at film scales 1/32 and 1/8): 9 blocks
-// 328 M / 428 M, 16 blocks 311 M / 405 M (another run: 9, 10, 12 blocks 350 / 350 /
-// 345 M and 448 / 447 / 443 M) -- unlike the single-scene kernels, these
-// grids lose more to their spills (the scene constants come from shared memory) than
-// they gain from the extra warps.
+// Resident blocks per SM (in blocks of 128 threads) of the class-specialised batched grids:
+// 64 random stones of 16 to 64 pixels a side, 9 / 12 / 16 blocks: 28.3 / 27.9 / 32.4 ms.
 #ifndef GR_BATCH_MIN_BLOCKS
-#define GR_BATCH_MIN_BLOCKS 9
+#define GR_BATCH_MIN_BLOCKS 12
 #endif
 
 namespace grh {
 
 gr_status launch_batch_class(int K, const grd::SceneSlot *slots, const grd::BatchSegment *segs, uint32_t n_segs,
-                             grd::Path *park, unsigned int *counts, uint64_t blocks, uint64_t park_blocks, size_t smem,
+                             uint32_t chunk, grd::Path *park, unsigned int *counts, uint64_t blocks, uint64_t park_blocks, size_t smem,
                              cudaStream_t s) {
     constexpr int IC = grd::K_ISO | grd::K_CLEAR;
     constexpr int MB = GR_BATCH_MIN_BLOCKS;
 #define GR_BATCH_CASE(KK)                                                                                       \
     case KK:                                                                                                    \
-        grd::launch_batch_grids<false, KK, MB>(slots, segs, n_segs, park, counts, blocks, park_blocks, smem, s); \
+        grd::launch_batch_grids<false, KK, MB>(slots, segs, n_segs, chunk, park, counts, blocks, park_blocks, smem, \
+                                               s);                                                              \
         break;
     switch (K) {
         GR_BATCH_CASE(IC | grd::k_env(GR_ENV_UNIFORM))

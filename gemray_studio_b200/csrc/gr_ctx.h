@@ -28,8 +28,8 @@ gr_status fail(gr_status st, const char *fmt, ...);
     } while (0)
 
 // Bounce caps of the staged kernels' first two stages ({0, 0} = the built-in pair) and
-// the resident blocks per SM their register allocation targets (0 = the built-in
-// kBuiltinScheduleBlocks): a staged schedule.
+// the resident blocks per SM their register allocation targets (0 =
+// builtin_schedule_blocks): a staged schedule.
 struct StageCaps {
     uint32_t first = 0, second = 0;
     uint32_t blocks = 0;
@@ -43,8 +43,13 @@ struct StageCaps {
 // spilled values.
 constexpr int kScheduleBlockCount = 4;
 constexpr uint32_t kScheduleBlocks[kScheduleBlockCount] = {9, 10, 12, 16};
-// The blocks per SM of a staged launch whose schedule is still open.
-constexpr uint32_t kBuiltinScheduleBlocks = 16;
+// The blocks per SM of a pooled launch whose schedule is still open: 16 for the clear
+// isotropic kernels (brilliant at 32 spp, 9 / 12 / 16 blocks: 42.3 / 39.0 / 37.6 ms), 12 for
+// the general ones, which spill more (emerald at 32 spp 40.1 / 38.7 / 41.3, tourmaline 2.43 /
+// 2.39 / 2.51).
+constexpr uint32_t builtin_schedule_blocks(int scene_class) {
+    return scene_class >= 0 && (scene_class & 2 /* grd::K_CLEAR */) ? 16u : 12u;
+}
 // Stage-cap pairs a stone chooses between: the pair measured best on the c2 brilliant
 // (long, TIR-trapped diamond paths), the one measured best on the c3 emerald (n ~ 1.6,
 // shorter paths; 3.9% faster there) and a longer pair for longer paths still.
@@ -208,7 +213,7 @@ namespace grh {
 // The two trace grids of a batched launch whose segments all have scene class K
 // (gr_batch_classes.cu); K is a clear-isotropic or general class with its environment.
 gr_status launch_batch_class(int K, const grd::SceneSlot *slots, const grd::BatchSegment *segs, uint32_t n_segs,
-                             grd::Path *park, unsigned int *counts, uint64_t blocks, uint64_t park_blocks, size_t smem,
+                             uint32_t chunk, grd::Path *park, unsigned int *counts, uint64_t blocks, uint64_t park_blocks, size_t smem,
                              cudaStream_t s);
 // Scene checks and encoding (gr_host.cu): validate, encode the constants, and upload
 // the scene's arrays into the context's buffers (prepare does all three).
@@ -225,13 +230,16 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
 // isotropic stones (K_ISO | K_CLEAR) and the rest, each with its environment kind;
 // -1 for scenes the extension variant handles (frosted, scattering, biaxial).
 int scene_class(const SceneConst &S);
-// Park buffers and caps of a staged single-scene launch (prepared by launch_trace).
+// Park buffers, counters and schedule of a pooled single-scene trace (prepared by
+// launch_trace).
 struct StagedLaunch {
     grd::Path *park1, *park2;
-    unsigned int *counts;
-    uint64_t cap1, cap2;
+    unsigned int *counts;      // parked paths of stages 1 and 2, zeroed
+    unsigned long long *work;  // items claimed by stages 1 to 3, zeroed
+    uint64_t cap1, cap2;       // park slots
     uint32_t cap_first, cap_second;
-    uint32_t blocks;  // kScheduleBlocks entry, 0 = kBuiltinScheduleBlocks
+    uint32_t blocks;  // kScheduleBlocks entry, 0 = builtin_schedule_blocks
+    int sm_count;
 };
 // The plain kernel (st == NULL) or the three staged launches of scene class K
 // (gr_single_clear.cu / gr_single_general.cu).
@@ -268,10 +276,11 @@ StageCapTune &accum_tune(gr_ctx *ctx, const gr_scene *sc);
 // The gr_accumulate tuning key of a scene (its stone, not its view).
 uint64_t stone_key(const gr_scene *sc);
 int trace_kernel_launches(int mode, const SceneConst &S, uint64_t n_tuples);
-// Park slots of a staged launch's first stage (1/8 of its tuples, at least 1,024, at
-// most 4 GiB of records), and the park buffer bytes of both capped stages.
-uint64_t staged_park_slots(uint64_t n_tuples);
-size_t staged_park_bytes(uint64_t n_tuples);
+// Park slots of a pooled trace of n_tuples tuples on sm_count SMs: what its resident threads
+// can hold, since only a draining pool parks; and the bytes of the park buffer (a header of
+// counters and both stages' records).
+uint64_t staged_park_slots(uint64_t n_tuples, int sm_count);
+size_t staged_park_bytes(uint64_t n_tuples, int sm_count);
 gr_status launch_fold(const float *xyz, uint32_t n_pixels, uint32_t spp, uint32_t first_pixel, float *film,
                       uint32_t kahan, cudaStream_t stream);
 }  // namespace grh

@@ -26,6 +26,7 @@
 #include "gr_ctx.h"
 #include "gr_host.h"
 #include "gr_kernels.cuh"
+#include "gr_single.cuh"
 
 using grd::SceneConst;
 
@@ -459,17 +460,17 @@ int trace_kernel_launches(int mode, const SceneConst &S, uint64_t n_tuples) {
     return staged ? 3 : 1;  // stages 1, 2 and 3
 }
 
-uint64_t staged_park_slots(uint64_t n_tuples) {
-    uint64_t cap1 = (n_tuples + 7) / 8;
-    const uint64_t max_cap = (4ull << 30) / sizeof(grd::Path);
-    if (cap1 > max_cap) cap1 = max_cap;
-    if (cap1 < 1024) cap1 = 1024;
-    return cap1;
+uint64_t staged_park_slots(uint64_t n_tuples, int sm_count) {
+    const uint64_t resident = (uint64_t)(sm_count > 0 ? sm_count : 1) * 2048u;  // threads per SM
+    return std::max<uint64_t>(1, std::min(n_tuples, resident));
 }
 
-size_t staged_park_bytes(uint64_t n_tuples) {
-    const uint64_t cap1 = staged_park_slots(n_tuples);
-    return (size_t)(cap1 + (cap1 + 3) / 4) * sizeof(grd::Path) + 256;
+// The park buffer's header: parked counts at 0, the sorted kernel's tuple counter at 8, the
+// pooled stages' item counters at 64.
+constexpr size_t kParkHeader = 256, kParkWork = 64;
+
+size_t staged_park_bytes(uint64_t n_tuples, int sm_count) {
+    return 2 * (size_t)staged_park_slots(n_tuples, sm_count) * sizeof(grd::Path) + kParkHeader;
 }
 
 // Trace tuples [0, R.n_tuples) of one chunk into xyz (device).
@@ -513,36 +514,25 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
         return launch_single_clear(K, S, B, R, xyz, stream, nullptr, (unsigned int *)pk.ptr + 2, ctx->sm_count);
     }
     if (mode == GR_KERNEL_STAGED) {
-        // park buffers: stage 1 parks up to 1/8 of the launch's paths (at most 4 GiB),
-        // stage 2 up to 1/4 of that; overflowing paths finish where they are
-        const uint64_t cap1 = staged_park_slots(R.n_tuples);
-        const uint64_t cap2 = caps.second == 0xFFFFFFFFu ? 0 : (cap1 + 3) / 4;
+        const uint64_t slots = staged_park_slots(R.n_tuples, ctx->sm_count);
         grh::DeviceBuffer &pk = park_buf ? *park_buf : ctx->park;
-        gr_status st = pk.reserve((size_t)(cap1 + cap2) * sizeof(grd::Path) + 256);
+        gr_status st = pk.reserve(staged_park_bytes(R.n_tuples, ctx->sm_count));
         if (st != GR_OK) return st;
-        unsigned int *counts = (unsigned int *)pk.ptr;
-        grd::Path *park1 = (grd::Path *)((char *)pk.ptr + 256);
-        grd::Path *park2 = park1 + cap1;
-        GR_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned int), stream));
-        if (!extras) {
-            const StagedLaunch sl{park1, park2, counts, cap1, cap2, caps.first, caps.second, caps.blocks};
+        GR_CUDA(cudaMemsetAsync(pk.ptr, 0, kParkHeader, stream));
+        StagedLaunch sl;
+        sl.counts = (unsigned int *)pk.ptr;
+        sl.work = (unsigned long long *)((char *)pk.ptr + kParkWork);
+        sl.park1 = (grd::Path *)((char *)pk.ptr + kParkHeader);
+        sl.park2 = sl.park1 + slots;
+        sl.cap1 = sl.cap2 = slots;
+        sl.cap_first = caps.first;
+        sl.cap_second = caps.second;
+        sl.blocks = caps.blocks;
+        sl.sm_count = ctx->sm_count > 0 ? ctx->sm_count : 1;
+        if (!extras)
             return clear ? launch_single_clear(K, S, B, R, xyz, stream, &sl)
                          : launch_single_general(K, S, B, R, xyz, stream, &sl);
-        }
-        const grd::ParkOut out1{park1, (uint32_t)cap1, counts};
-        const grd::ParkOut out2{park2, (uint32_t)cap2, counts + 1};
-        const grd::ParkOut none{nullptr, 0, nullptr};
-        const unsigned b2 = (unsigned)((cap1 + grd::TRACE_THREADS - 1) / grd::TRACE_THREADS);
-        const unsigned b3 = (unsigned)((cap2 + grd::TRACE_THREADS - 1) / grd::TRACE_THREADS);
-        {
-            grd::k_trace_stage1<true><<<(unsigned)plain_blocks, grd::TRACE_THREADS, smem, stream>>>(S, B, R, xyz, out1,
-                                                                                                  caps.first);
-            grd::k_trace_stage2<true><<<b2, grd::TRACE_THREADS, smem, stream>>>(S, B, park1, (uint32_t)cap1, counts,
-                                                                                caps.second, out2, xyz);
-            if (cap2)
-                grd::k_trace_stage2<true><<<b3, grd::TRACE_THREADS, smem, stream>>>(S, B, park2, (uint32_t)cap2,
-                                                                                    counts + 1, 0xFFFFFFFFu, none, xyz);
-        }
+        grd::launch_pool<true, grd::K_ANY, GR_TRACE_MIN_BLOCKS>(S, B, R, xyz, stream, pool_launch(sl));
         GR_CUDA(cudaGetLastError());
         return GR_OK;
     }

@@ -48,6 +48,14 @@ __device__ __forceinline__ void tuple_coords(const LaunchRange &R, uint64_t t, u
 }
 
 
+// A finished path's sample into its tuple's place.
+__device__ __forceinline__ void store_sample(float *__restrict__ xyz, const Path &P, V3 c) {
+    const uint64_t t = p_tuple(P);
+    xyz[3 * t + 0] = c.x;
+    xyz[3 * t + 1] = c.y;
+    xyz[3 * t + 2] = c.z;
+}
+
 // One warp folds pixel `px` (local to its xyz block) into film pixel `film_pixel`.
 // Add mode (cont == 0): the samples are summed in order from zero and the sum is
 // added to the film once -- the reference's per-call semantics.  Continue mode

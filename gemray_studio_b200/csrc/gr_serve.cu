@@ -759,7 +759,7 @@ ServeState *serve_state(gr_ctx *ctx) {
                     continue;
                 }
                 L->xyz.reserve((size_t)kClassTuples[c] * 12);
-                L->park.reserve(grh::staged_park_bytes(kClassTuples[c]));
+                L->park.reserve(grh::staged_park_bytes(kClassTuples[c], ctx->sm_count));
                 ctx->serve->lanes.push_back(L);
             }
         }

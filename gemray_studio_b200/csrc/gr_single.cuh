@@ -9,30 +9,23 @@
 
 namespace grh {
 
-// The three staged launches at MB blocks per SM.
+inline grd::PoolLaunch pool_launch(const StagedLaunch &st) {
+    return grd::PoolLaunch{st.park1, st.park2, (uint32_t)st.cap1, (uint32_t)st.cap2, st.counts, st.work,
+                           st.cap_first, st.cap_second, st.sm_count};
+}
+
+// The three pooled launches at MB blocks per SM.
 template <int K, int MB>
 gr_status launch_staged_mb(const SceneConst &S, const grd::SceneBuffers &B, const grd::LaunchRange &R, float *xyz,
                            cudaStream_t stream, const StagedLaunch *st) {
-    const size_t smem = grd::planes_smem_bytes(S.n_planes);
-    const unsigned blocks = (unsigned)((R.n_tuples + grd::TRACE_THREADS - 1) / grd::TRACE_THREADS);
-    const grd::ParkOut out1{st->park1, (uint32_t)st->cap1, st->counts};
-    const grd::ParkOut out2{st->park2, (uint32_t)st->cap2, st->counts + 1};
-    const grd::ParkOut none{nullptr, 0, nullptr};
-    const unsigned b2 = (unsigned)((st->cap1 + grd::TRACE_THREADS - 1) / grd::TRACE_THREADS);
-    const unsigned b3 = (unsigned)((st->cap2 + grd::TRACE_THREADS - 1) / grd::TRACE_THREADS);
-    grd::k_trace_stage1<false, K, MB><<<blocks, grd::TRACE_THREADS, smem, stream>>>(S, B, R, xyz, out1, st->cap_first);
-    grd::k_trace_stage2<false, K, MB><<<b2, grd::TRACE_THREADS, smem, stream>>>(
-        S, B, st->park1, (uint32_t)st->cap1, st->counts, st->cap_second, out2, xyz);
-    if (st->cap2)
-        grd::k_trace_stage2<false, K, MB><<<b3, grd::TRACE_THREADS, smem, stream>>>(
-            S, B, st->park2, (uint32_t)st->cap2, st->counts + 1, 0xFFFFFFFFu, none, xyz);
+    grd::launch_pool<false, K, MB>(S, B, R, xyz, stream, pool_launch(*st));
     GR_CUDA(cudaGetLastError());
     return GR_OK;
 }
 
 // The plain kernel (st == NULL, at the built-in GR_TRACE_MIN_BLOCKS), or the staged
 // launches at the blocks per SM the schedule asks for (kScheduleBlocks; 0 =
-// kBuiltinScheduleBlocks).
+// builtin_schedule_blocks).
 template <int K>
 gr_status launch_single_k(const SceneConst &S, const grd::SceneBuffers &B, const grd::LaunchRange &R, float *xyz,
                           cudaStream_t stream, const StagedLaunch *st) {
@@ -45,7 +38,7 @@ gr_status launch_single_k(const SceneConst &S, const grd::SceneBuffers &B, const
         return GR_OK;
     }
     static_assert(kScheduleBlockCount == 4, "one launch per kScheduleBlocks entry");
-    switch (st->blocks ? st->blocks : kBuiltinScheduleBlocks) {
+    switch (st->blocks ? st->blocks : builtin_schedule_blocks(K)) {
         case kScheduleBlocks[0]: return launch_staged_mb<K, kScheduleBlocks[0]>(S, B, R, xyz, stream, st);
         case kScheduleBlocks[1]: return launch_staged_mb<K, kScheduleBlocks[1]>(S, B, R, xyz, stream, st);
         case kScheduleBlocks[2]: return launch_staged_mb<K, kScheduleBlocks[2]>(S, B, R, xyz, stream, st);

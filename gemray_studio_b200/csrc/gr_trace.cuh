@@ -74,6 +74,7 @@ constexpr uint32_t F_ABSORBING = 1u << 2;
 constexpr uint32_t F_ESCAPED = 1u << 3;
 constexpr uint32_t F_ALIVE = 1u << 4;
 constexpr uint32_t F_TIR = 1u << 5;  // the pending event is a hero TIR
+constexpr uint32_t F_NONE = 1u << 6;  // no path: a thread past the launch's tuples
 constexpr uint32_t BOUNCE_SHIFT = 8;  // 13 bits: bounce index, at most GR_MAX_BOUNCES
 constexpr uint32_t BOUNCE_MASK = 0x1FFFu;
 constexpr uint32_t LIVE_SHIFT = 21;   // 8 bits: the channels that still carry light
@@ -347,10 +348,9 @@ __device__ __forceinline__ bool intersect(const float4 *__restrict__ planes, uin
 // Planes are staged twice in shared memory: as float4 (n.xyz, d) for lookups by
 // index, and pair-interleaved as {nx0, nx1, ny0, ny1}, {nz0, nz1, d0, d1}, so that
 // one packed mul.rn.f32x2 (sm_100: two IEEE round-to-nearest products) forms the
-// same product for two planes.  The sums stay scalar: a fully packed evaluation
-// (packed sums as well) did not reproduce the scalar scan's results on B200, while
-// packed products with scalar sums are bit-identical to it.  An odd tail is padded
-// with the plane n = 0, d = -1 (denom = 0, side = -1), which never acts.
+// same product for two planes.  The general scan keeps its sums scalar; the interior
+// scan packs them too (add2).  An odd tail is padded with the plane n = 0,
+// d = -1 (denom = 0, side = -1), which never acts.
 //
 // The per-plane decisions are those of the reference loop, reduced by two exact
 // rules (intersect.rs:93-132):
@@ -385,6 +385,15 @@ __device__ __forceinline__ void upk2(f32x2 v, float &lo, float &hi) {
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// The sum of two pairs, each rounded once: a * one + b with a pair of ones that ptxas does
+// not know.  Written as add.rn.f32x2, ptxas contracts it with the product that feeds it into
+// one rounding (about one path in 7e9 then takes another facet than the reference's).
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b, f32x2 one) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(one), "l"(b));
     return r;
 }
 
@@ -428,6 +437,66 @@ __device__ __forceinline__ bool scan_plane(float denom, float side, int i, float
         }
     }
     return true;
+}
+
+// The scan of a ray inside the stone, without branches: the exit facet of a ray whose
+// origin has side < 0 for every plane.  Then no plane is outside or entered (an entering
+// plane with side < 0 has t < 0), so the clip is the least t = -side / denom over the
+// planes with denom > 1e-7, and 1 / t orders them: v = denom * rcp(side) = -1 / t is
+// negative for exactly those planes, and the exit facet has the least v.  v carries the
+// plane's index in its low 9 bits, so one minimum finds both, and the second least v
+// says whether the order is certain: rcp.approx (1 ulp), the product and the 9 bits
+// move v by less than 2^-13.9 of itself, so when the second is not within 2^-11 of the
+// least, the winner's exact quotient is the strictly least one whatever the rounding.
+// Only that quotient is then divided, from the same sums as the reference.
+// Everything else -- a side that is not clearly negative (the origin on or outside a
+// plane, a NaN), no plane to leave through, two facets within 2^-11 (an edge) -- returns
+// SCAN_UNDECIDED, and the general scan decides.
+//
+// Why: the general scan's updates and divisions are branches, and among the lanes of a
+// warp some lane takes them at nearly every plane, so the warp pays for them 73 times a
+// bounce; this scan issues 14 instructions per plane whatever the lanes do.
+constexpr int SCAN_MISS = 0, SCAN_HIT = 1, SCAN_UNDECIDED = 2;
+constexpr uint32_t SCAN_INDEX_MASK = GR_MAX_PLANES - 1u;
+static_assert((GR_MAX_PLANES & (GR_MAX_PLANES - 1)) == 0 && GR_MAX_PLANES <= 512, "the index fits the key's low 9 bits");
+
+__device__ __forceinline__ float scan_key(float v, uint32_t i) {
+    return __uint_as_float((__float_as_uint(v) & ~SCAN_INDEX_MASK) | i);
+}
+
+#ifndef GR_SCAN_UNROLL
+#define GR_SCAN_UNROLL 1
+#endif
+constexpr int SCAN_UNROLL = GR_SCAN_UNROLL;
+__device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, float &t_hit, int &idx_hit) {
+    const f32x2 dx = pk2(d.x, d.x), dy = pk2(d.y, d.y), dz = pk2(d.z, d.z);
+    const f32x2 ox = pk2(o.x, o.x), oy = pk2(o.y, o.y), oz = pk2(o.z, o.z);
+    const uint32_t n2 = (PL.n + 1u) & ~1u;
+    const float unit = __uint_as_float(0x3f800000u | (PL.n >> 16));  // 1.0f: n <= GR_MAX_PLANES
+    const f32x2 one = pk2(unit, unit);
+    float best = 3.0e38f, second = 3.0e38f, side_max = -3.0e38f;
+#pragma unroll SCAN_UNROLL
+    for (uint32_t i = 0; i < n2; i += 2) {
+        const float4 a = PL.pairs[i], b = PL.pairs[i + 1];
+        const f32x2 nx = pk2(a.x, a.y), ny = pk2(a.z, a.w), nz = pk2(b.x, b.y);
+        float den0, den1, sid0, sid1;
+        upk2(add2(add2(mul2(nx, dx), mul2(ny, dy), one), mul2(nz, dz), one), den0, den1);
+        upk2(add2(add2(add2(mul2(nx, ox), mul2(ny, oy), one), mul2(nz, oz), one), pk2(b.z, b.w), one), sid0, sid1);
+        side_max = fmaxf(side_max, fmaxf(sid0, sid1));
+        const float k0 = scan_key(den0 * rcp_approx(sid0), i), k1 = scan_key(den1 * rcp_approx(sid1), i + 1u);
+        const float lo = fminf(k0, k1), hi = fmaxf(k0, k1);
+        second = fminf(fminf(second, hi), fmaxf(best, lo));
+        best = fminf(best, lo);
+    }
+    if (!(side_max < -1e-30f) || !(best < -1e-20f) || !(second > best * (1.0f - 4.8828125e-4f))) return SCAN_UNDECIDED;
+    const int idx = (int)(__float_as_uint(best) & SCAN_INDEX_MASK);
+    const float4 p = PL.aos[idx];
+    const float denom = (p.x * d.x + p.y * d.y) + p.z * d.z;
+    const float side = p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z);
+    if (!(denom > 1e-7f)) return SCAN_UNDECIDED;
+    t_hit = (-side) / denom;
+    idx_hit = idx;
+    return t_hit > 1e-4f ? SCAN_HIT : SCAN_MISS;
 }
 
 // The reference clip (intersect.rs:93-132) in FP64, t rounded back to f32: the
@@ -507,6 +576,17 @@ __device__ __forceinline__ bool intersect(const Planes &PL, V3 o, V3 d, float &t
         return true;
     }
     return false;
+}
+
+// The clip of a ray that may start anywhere, its origin taken to be inside first
+// (`inside`): the interior scan, and the general one where that does not decide.
+template <bool R = false>
+__device__ __forceinline__ bool intersect_from(const Planes &PL, bool inside, V3 o, V3 d, float &t_hit, int &idx_hit) {
+    if (!R && inside) {
+        const int r = intersect_inside(PL, o, d, t_hit, idx_hit);
+        if (r != SCAN_UNDECIDED) return r == SCAN_HIT;
+    }
+    return intersect<R>(PL, o, d, t_hit, idx_hit);
 }
 
 __device__ __forceinline__ V3 plane_normal(const float4 *planes, int idx) {
@@ -736,31 +816,40 @@ __device__ __forceinline__ float theta_c(V3 kk, V3 normal, float cos_i, float on
     return theta;
 }
 
-// One intersection and everything of the bounce up to the hero's event decision
+// One bounce is step_scan (the intersection), step_facet (everything up to the hero's event
+// decision) and then step_reflect or step_refract; step_hit is the first two together.
+//
+// step_scan: false on an escape (F_ESCAPED set, F_ALIVE cleared; accumulate_miss_radiance,
+// transport.rs:67-90, runs in path_finish).
+template <class CT, bool R = false>
+__device__ __forceinline__ bool step_scan(Path &P, const Planes &PL, float &t_hit, int &fidx, CT &ct) {
+    const uint32_t bits = state_bits(P);
+    const V3 o = xyz(P.o_hero), d = xyz(P.d_seed);
+    tally(ct, C_BOUNCES);
+    if (!intersect_from<R>(PL, (bits & F_INSIDE) != 0, o, d, t_hit, fidx)) {
+        tally(ct, C_ESCAPES);
+        note_end(ct, bits_bounce(bits), GR_TERM_ESCAPED);
+        set_state_bits(P, (bits | F_ESCAPED) & ~F_ALIVE);
+        return false;
+    }
+    note_hit(ct, bits_bounce(bits), fidx, t_hit);
+    return true;
+}
+
+// Everything of the bounce between the hit and the hero's event decision
 // (transport.rs:781-895, raytracer/absorption.rs:71-141, refraction.rs:428-547,
-// 1036-1060).  Returns EV_DONE on an escape (F_ESCAPED set, F_ALIVE cleared).
+// 1036-1060).
 // X: the instantiation that handles frosted facets, volume scattering and biaxial
 // materials (scenes without any of them run the X = false code, which has none of
 // those branches).
 template <int U, class CT, bool R = false, bool X = false, int K = K_ANY>
-__device__ __forceinline__ uint32_t step_hit(Path &P, const SceneConst &S, const SceneBuffers &B, const Planes &PL,
-                                             Event &E, CT &ct) {
+__device__ __forceinline__ uint32_t step_facet(Path &P, const SceneConst &S, const SceneBuffers &B, const Planes &PL,
+                                               float t_hit, int fidx, Event &E, CT &ct) {
     uint32_t bits = state_bits(P);
     const uint32_t bounce = bits_bounce(bits);
     const bool inside = (bits & F_INSIDE) != 0;
     const uint32_t live = live_channels<CT, X>(bits);
     const V3 o = xyz(P.o_hero), d = xyz(P.d_seed), kk = xyz(P.k_state);
-    float t_hit = 0.0f;
-    int fidx = 0;
-    tally(ct, C_BOUNCES);
-    if (!intersect<R>(PL, o, d, t_hit, fidx)) {
-        // accumulate_miss_radiance (transport.rs:67-90) runs in path_finish
-        tally(ct, C_ESCAPES);
-        note_end(ct, bounce, GR_TERM_ESCAPED);
-        set_state_bits(P, (bits | F_ESCAPED) & ~F_ALIVE);
-        return EV_DONE;
-    }
-    note_hit(ct, bounce, fidx, t_hit);
     if (bounce == 0) {  // the bounce index grows with every event: the first hit, once per path
         bits |= channel_tables<U, X, K>(P, S, B);
         set_state_bits(P, bits);
@@ -876,6 +965,15 @@ __device__ __forceinline__ uint32_t step_hit(Path &P, const SceneConst &S, const
     return refract ? EV_REFRACT : EV_REFLECT;
 }
 
+template <int U, class CT, bool R = false, bool X = false, int K = K_ANY>
+__device__ __forceinline__ uint32_t step_hit(Path &P, const SceneConst &S, const SceneBuffers &B, const Planes &PL,
+                                             Event &E, CT &ct) {
+    float t_hit = 0.0f;
+    int fidx = 0;
+    if (!step_scan<CT, R>(P, PL, t_hit, fidx, ct)) return EV_DONE;
+    return step_facet<U, CT, R, X, K>(P, S, B, PL, t_hit, fidx, E, ct);
+}
+
 // Direction / state update after an event, internal mode coupling and Russian
 // roulette (transport.rs:177-193,204-220,343-353,919-928).
 template <class CT, int K = K_ANY, bool X = false>
@@ -915,6 +1013,19 @@ __device__ __forceinline__ void step_post(Path &P, const SceneConst &S, V3 hp, V
     bits = (bits & ~(BOUNCE_MASK << BOUNCE_SHIFT)) | (nb << BOUNCE_SHIFT);
     if (nb >= S.max_bounces) bits &= ~F_ALIVE;
     set_state_bits(P, bits);
+}
+
+// A ray outside the stone that starts beyond the plane of the facet it just met and does not
+// enter it misses: the clip's test of that one plane (scan_plane), which ends the scan
+// whatever the other planes say.  So a path that leaves ends here, one scan early.
+__device__ __forceinline__ void step_leave(Path &P, const Planes &PL, int fidx) {
+    const uint32_t bits = state_bits(P);
+    if ((bits & (F_ALIVE | F_INSIDE)) != F_ALIVE || fidx < 0) return;
+    const float4 p = PL.aos[fidx];
+    const V3 o = xyz(P.o_hero), d = xyz(P.d_seed);
+    const float denom = (p.x * d.x + p.y * d.y) + p.z * d.z;
+    const float side = p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z);
+    if (!(denom < -1e-7f) && side > 0.0f) set_state_bits(P, (bits | F_ESCAPED) & ~F_ALIVE);
 }
 
 // apply_frosted_bounce (raytracer/scattering.rs:522-602): a Lambertian lobe on either

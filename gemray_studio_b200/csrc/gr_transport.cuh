@@ -47,51 +47,69 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_plain(SceneConst S,
     }
 }
 
-// Staged kernels (the scheme and run_or_park are in gr_stage.cuh).
-// MB: resident blocks per SM the register allocation targets (the schedule tuner's
-// warps-per-SM dimension).
+// Pooled kernels (the scheme and run_pool are in gr_stage.cuh), three launches per trace:
+// k_trace_pool over the launch's tuples, then k_trace_resume over the paths it parked past
+// the first cap and again over those parked past the second, to their ends.
+// MB: resident blocks per SM the register allocation targets, in blocks of 128 threads (the
+// schedule tuner's dimension).  work: the launch's zeroed tuple counter.
 template <bool EXTRAS, int K = K_ANY, int MB = GR_TRACE_MIN_BLOCKS>
-__global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_stage1(SceneConst S, SceneBuffers B,
-                                                                                     LaunchRange R,
-                                                                                     float *__restrict__ xyz,
-                                                                                     ParkOut out, uint32_t bounce_cap) {
+__global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, pool_threads<EXTRAS, K>()))
+    k_trace_pool(SceneConst S, SceneBuffers B, LaunchRange R, float *__restrict__ xyz, unsigned long long *work,
+                 ParkOut out, uint32_t bounce_cap) {
     extern __shared__ float4 s_planes[];
     const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = t < R.n_tuples;
     Path P;
-    if (active) {
-        uint32_t pixel, sample;
-        tuple_coords(R, t, pixel, sample);
-        path_init<K>(P, S, pixel, sample, (uint32_t)t);
-    }
-    if (run_or_park<EXTRAS, K>(P, S, B, PL, active, bounce_cap, out) || !active) return;
-    const V3 c = path_finish<1, false, K, EXTRAS>(P, S, B);
-    xyz[3 * t + 0] = c.x;
-    xyz[3 * t + 1] = c.y;
-    xyz[3 * t + 2] = c.z;
+    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K>(
+        P, S, B, PL, PoolQueue{work, R.n_tuples}, bounce_cap, out,
+        [&](Path &q, uint64_t t) {
+            uint32_t pixel, sample;
+            tuple_coords(R, t, pixel, sample);
+            path_init<K>(q, S, pixel, sample, (uint32_t)t);
+        },
+        [&](const Path &q) { store_sample(xyz, q, path_finish<1, false, K, EXTRAS>(q, S, B)); });
 }
 
-// Continuation: parked paths [0, min(*count_in, cap_in)) resumed one per thread, up to
-// `bounce_cap`, survivors parked in `out` (out.cap 0: run to the end).
+// Parked paths [0, min(*count_in, cap_in)), up to `bounce_cap`, survivors parked in `out`
+// (out.cap 0: to the end).
 template <bool EXTRAS, int K = K_ANY, int MB = GR_TRACE_MIN_BLOCKS>
-__global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_stage2(
-    SceneConst S, SceneBuffers B, const Path *__restrict__ park_in, uint32_t cap_in,
-    const unsigned int *__restrict__ count_in, uint32_t bounce_cap, ParkOut out, float *__restrict__ xyz) {
+__global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, pool_threads<EXTRAS, K>()))
+    k_trace_resume(SceneConst S, SceneBuffers B, const Path *__restrict__ park_in, uint32_t cap_in,
+                   const unsigned int *__restrict__ count_in, uint32_t bounce_cap, unsigned long long *work, ParkOut out,
+                   float *__restrict__ xyz) {
     const uint32_t n = min((uint32_t)*count_in, cap_in);
-    if ((uint64_t)blockIdx.x * blockDim.x >= n) return;  // whole block past the parked paths
+    if ((uint64_t)blockIdx.x * blockDim.x >= n) return;  // more blocks than parked paths fill
     extern __shared__ float4 s_planes[];
     const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < n;
     Path P;
-    if (active) P = park_in[i];
-    if (run_or_park<EXTRAS, K>(P, S, B, PL, active, bounce_cap, out) || !active) return;
-    const V3 c = path_finish<1, false, K, EXTRAS>(P, S, B);
-    const uint64_t t = p_tuple(P);
-    xyz[3 * t + 0] = c.x;
-    xyz[3 * t + 1] = c.y;
-    xyz[3 * t + 2] = c.z;
+    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K>(
+        P, S, B, PL, PoolQueue{work, n}, bounce_cap, out,
+        [&](Path &q, uint64_t i) { copy_record<record_rows<EXTRAS, K>()>(q, park_in[i]); },
+        [&](const Path &q) { store_sample(xyz, q, path_finish<1, false, K, EXTRAS>(q, S, B)); });
+}
+
+// The three launches of a pooled trace (`work`: three zeroed counters, one per stage; `grid`
+// blocks at most, as many as stay resident).
+struct PoolLaunch {
+    Path *park1, *park2;
+    uint32_t cap1, cap2;  // slots
+    unsigned int *counts;
+    unsigned long long *work;
+    uint32_t cap_first, cap_second;
+    int sm_count;
+};
+template <bool EXTRAS, int K, int MB>
+void launch_pool(const SceneConst &S, const SceneBuffers &B, const LaunchRange &R, float *xyz, cudaStream_t stream,
+                 const PoolLaunch &L) {
+    constexpr int T = pool_threads<EXTRAS, K>();
+    const size_t smem = planes_smem_bytes(S.n_planes);
+    const uint64_t resident = (uint64_t)L.sm_count * pool_blocks(MB, T), need = (R.n_tuples + T - 1) / T;
+    const unsigned grid = (unsigned)(need < resident ? need : resident);
+    const ParkOut out1{L.park1, L.cap1, L.counts}, out2{L.park2, L.cap2, L.counts + 1}, none{nullptr, 0, nullptr};
+    k_trace_pool<EXTRAS, K, MB><<<grid, T, smem, stream>>>(S, B, R, xyz, L.work, out1, L.cap_first);
+    k_trace_resume<EXTRAS, K, MB><<<grid, T, smem, stream>>>(S, B, L.park1, L.cap1, L.counts, L.cap_second, L.work + 1,
+                                                             out2, xyz);
+    k_trace_resume<EXTRAS, K, MB><<<grid, T, smem, stream>>>(S, B, L.park2, L.cap2, L.counts + 1, 0xFFFFFFFFu, L.work + 2,
+                                                             none, xyz);
 }
 
 }  // namespace grd

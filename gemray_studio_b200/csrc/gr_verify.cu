@@ -156,7 +156,7 @@ __global__ void k_intersect_rays(const float4 *__restrict__ planes, uint32_t n_p
     const float *r = rays + 6 * (size_t)i;
     float t = 0.0f;
     int idx = -1;
-    const bool hit = intersect<false>(PL, v3(r[0], r[1], r[2]), v3(r[3], r[4], r[5]), t, idx);
+    const bool hit = intersect_from<false>(PL, true, v3(r[0], r[1], r[2]), v3(r[3], r[4], r[5]), t, idx);
     t_out[i] = hit ? t : 0.0f;
     facet_out[i] = hit ? idx : -1;
 }

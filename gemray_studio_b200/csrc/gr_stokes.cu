@@ -9,44 +9,39 @@
 // gr_trace.cuh), folded per pixel in sample order like the XYZ film.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <vector>
 
 #include "gr_ctx.h"
-#include "gr_launch.cuh"
+#include "gr_stage.cuh"
 
 using grh::fail;
 
 namespace grd {
 
-// The plain kernel writing XYZ (the same arithmetic as k_trace_plain) and IQUV per tuple.
-template <bool EXTRAS>
-__global__ void __launch_bounds__(TRACE_THREADS, GR_TRACE_MIN_BLOCKS) k_trace_stokes(SceneConst S, SceneBuffers B,
-                                                                                     LaunchRange R,
-                                                                                     float *__restrict__ xyz,
-                                                                                     float4 *__restrict__ iquv) {
+// The pooled kernel (gr_stage.cuh) writing XYZ (the same arithmetic as the film's kernels) and
+// IQUV per tuple; nothing is parked.
+template <bool EXTRAS, int MB>
+__global__ void __launch_bounds__(pool_threads<EXTRAS, K_ANY>(), pool_blocks(MB, pool_threads<EXTRAS, K_ANY>()))
+    k_trace_stokes(SceneConst S, SceneBuffers B, LaunchRange R, float *__restrict__ xyz, float4 *__restrict__ iquv,
+                   unsigned long long *work) {
     extern __shared__ float4 s_planes[];
     const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= R.n_tuples) return;
-    uint32_t pixel, sample;
-    tuple_coords(R, t, pixel, sample);
     Path P;
-    path_init(P, S, pixel, sample, (uint32_t)t);
-    NoCounters nc;
-    while (state_bits(P) & F_ALIVE) {
-        Event E;
-        const uint32_t ev = step_hit<1, NoCounters, false, EXTRAS>(P, S, B, PL, E, nc);
-        if (ev == EV_REFLECT) step_reflect<1, NoCounters, EXTRAS>(P, S, E, nc);
-        else if (ev == EV_REFRACT) step_refract<1, NoCounters, EXTRAS>(P, S, E, nc);
-    }
-    float4 s4;
-    const V3 c = path_finish<1, true, K_ANY, EXTRAS>(P, S, B, &s4);
-    xyz[3 * t + 0] = c.x;
-    xyz[3 * t + 1] = c.y;
-    xyz[3 * t + 2] = c.z;
-    iquv[t] = s4;
+    run_pool<pool_threads<EXTRAS, K_ANY>(), EXTRAS, K_ANY>(
+        P, S, B, PL, PoolQueue{work, R.n_tuples}, 0xFFFFFFFFu, ParkOut{nullptr, 0, nullptr},
+        [&](Path &q, uint64_t t) {
+            uint32_t pixel, sample;
+            tuple_coords(R, t, pixel, sample);
+            path_init(q, S, pixel, sample, (uint32_t)t);
+        },
+        [&](const Path &q) {
+            float4 s4;
+            store_sample(xyz, q, path_finish<1, true, K_ANY, EXTRAS>(q, S, B, &s4));
+            iquv[p_tuple(q)] = s4;
+        });
 }
 
 // One warp per pixel: the pixel's spp Stokes vectors summed in sample order from zero,
@@ -75,6 +70,13 @@ __global__ void k_stokes_fold(const float4 *__restrict__ iquv, uint32_t n_pixels
 }
 
 }  // namespace grd
+
+// Resident blocks per SM of the Stokes kernels, in blocks of 128 threads (384 x 256 emerald at
+// 64 spp: one path per thread 15.8 ms; pooled at 12 / 9 blocks 7.69 / 7.83).
+#ifndef GR_STOKES_BLOCKS
+#define GR_STOKES_BLOCKS 12
+#endif
+constexpr int kStokesBlocks = GR_STOKES_BLOCKS;
 
 extern "C" {
 
@@ -112,6 +114,8 @@ gr_status gr_accumulate_stokes(gr_ctx *ctx, const gr_scene *sc, uint32_t sample_
     float *txyz = (float *)ctx->xyz.ptr;
     float4 *tiquv = (float4 *)((char *)ctx->xyz.ptr + toff);
     const size_t smem = grd::planes_smem_bytes(S.n_planes);
+    st = ctx->counter.reserve(64);
+    if (st != GR_OK) return st;
     for (uint64_t first = 0; first < n_pixels; first += chunk_pixels) {
         const uint64_t np = n_pixels - first < chunk_pixels ? n_pixels - first : chunk_pixels;
         grd::LaunchRange R;
@@ -120,11 +124,15 @@ gr_status gr_accumulate_stokes(gr_ctx *ctx, const gr_scene *sc, uint32_t sample_
         R.sample_offset = sample_offset;
         R.spp = spp;
         R.n_tuples = np * spp;
-        const unsigned blocks = (unsigned)((R.n_tuples + grd::TRACE_THREADS - 1) / grd::TRACE_THREADS);
+        constexpr int T = grd::pool_threads<true, grd::K_ANY>();
+        const uint64_t resident = (uint64_t)(ctx->sm_count > 0 ? ctx->sm_count : 1) * grd::pool_blocks(kStokesBlocks, T);
+        const unsigned blocks = (unsigned)std::min<uint64_t>(resident, (R.n_tuples + T - 1) / T);
+        GR_CUDA(cudaMemsetAsync(ctx->counter.ptr, 0, sizeof(unsigned long long), ctx->stream));
+        unsigned long long *work = (unsigned long long *)ctx->counter.ptr;
         if (grd::needs_extras(S))
-            grd::k_trace_stokes<true><<<blocks, grd::TRACE_THREADS, smem, ctx->stream>>>(S, B, R, txyz, tiquv);
+            grd::k_trace_stokes<true, kStokesBlocks><<<blocks, T, smem, ctx->stream>>>(S, B, R, txyz, tiquv, work);
         else
-            grd::k_trace_stokes<false><<<blocks, grd::TRACE_THREADS, smem, ctx->stream>>>(S, B, R, txyz, tiquv);
+            grd::k_trace_stokes<false, kStokesBlocks><<<blocks, T, smem, ctx->stream>>>(S, B, R, txyz, tiquv, work);
         GR_CUDA(cudaGetLastError());
         ctx->trace_launches += 1;
         st = grh::launch_fold(txyz, (uint32_t)np, spp, (uint32_t)first, film_x, (S.flags & GR_FLAG_KAHAN_FILM) ? 1u : 0u,

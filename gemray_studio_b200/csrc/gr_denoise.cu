@@ -15,6 +15,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <utility>
 
 #include "gr_ctx.h"
 #include "gr_launch.cuh"
@@ -57,25 +58,41 @@ __global__ void __launch_bounds__(128) k_guide_pass(SceneConst S, const float4 *
 
 __device__ __forceinline__ float sanitize(float v) { return isfinite(v) ? v : 0.0f; }
 
-// unit_normal_or_zero (:268-276), and the colour input scaled (accum * (1 / count) in
-// denoise_and_tonemap_frame) or copied.
-__global__ void k_denoise_prep(const float *__restrict__ normal, float *__restrict__ nn, const float *__restrict__ film,
-                               float *__restrict__ color, float inv_count, uint32_t scale, uint64_t n_px) {
+// The filter's per-pixel records, so that a tap is two 16-byte loads: colour and facet id,
+// unit normal and finite depth (unit_normal_or_zero, :268-276; the depth term sanitizes its
+// input).  The colour is the averaged image, or the film scaled (accum * (1 / count) in
+// denoise_and_tonemap_frame).  plain != NULL: the colour alone, for the identity filter.
+__global__ void __launch_bounds__(256) k_denoise_prep(const float *__restrict__ normal, const float *__restrict__ depth,
+                                                      const int32_t *__restrict__ facet, const float *__restrict__ film,
+                                                      float4 *__restrict__ color, float4 *__restrict__ guide,
+                                                      float *__restrict__ plain, float inv_count, uint32_t scale,
+                                                      uint64_t n_px) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_px) return;
+    V3 c = v3(film[3 * i], film[3 * i + 1], film[3 * i + 2]);
+    if (scale) c = mul(c, inv_count);
+    if (plain) {
+        plain[3 * i + 0] = c.x;
+        plain[3 * i + 1] = c.y;
+        plain[3 * i + 2] = c.z;
+        return;
+    }
     const V3 n = v3(sanitize(normal[3 * i]), sanitize(normal[3 * i + 1]), sanitize(normal[3 * i + 2]));
     const float l = sqrtf(dot(n, n));
     const bool z = l <= 1.0e-8f;
-    nn[3 * i + 0] = z ? 0.0f : n.x / l;
-    nn[3 * i + 1] = z ? 0.0f : n.y / l;
-    nn[3 * i + 2] = z ? 0.0f : n.z / l;
-    if (film) {
-        for (int c = 0; c < 3; ++c) color[3 * i + c] = scale ? film[3 * i + c] * inv_count : film[3 * i + c];
-    }
+    color[i] = make_float4(c.x, c.y, c.z, __int_as_float(facet[i]));
+    guide[i] = make_float4(z ? 0.0f : n.x / l, z ? 0.0f : n.y / l, z ? 0.0f : n.z / l, sanitize(depth[i]));
 }
 
 // cos_pow (:294-311): repeated squaring for power-of-two integer exponents, else powf.
-__device__ __forceinline__ float cos_pow(float base, float power, uint32_t squarings, bool pow2) {
+// SQ: the number of squarings where it is known at compile time (the default power 64: 6).
+template <int SQ> __device__ __forceinline__ float cos_pow(float base, float power, uint32_t squarings, bool pow2) {
+    if (SQ > 0) {
+        float v = base;
+#pragma unroll
+        for (int k = 0; k < SQ; ++k) v *= v;
+        return v;
+    }
     if (pow2) {
         float v = base;
         for (uint32_t k = 0; k < squarings; ++k) v *= v;
@@ -90,54 +107,68 @@ struct AtrousConst {
     uint32_t squarings, pow2;
 };
 
-__global__ void __launch_bounds__(128) k_atrous_pass(AtrousConst A, const float *__restrict__ src,
-                                                     float *__restrict__ dst, const float *__restrict__ depth,
-                                                     const float *__restrict__ nn, const int32_t *__restrict__ facet,
-                                                     int stride) {
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= (uint64_t)A.w * A.h) return;
-    const int64_t y = (int64_t)(c / A.w), x = (int64_t)(c % A.w);
+// One pass, a thread per output pixel, 32 x 8 pixels per block (the rows of the block's taps
+// overlap in L1).  Bound by issue: ~25 taps of ~60 instructions, two of them accurate expf.
+// Separate 12-byte colour and normal images, depth and facet loads and 64-bit index
+// arithmetic took 275 us a pass at 1920x1080, the two records per tap 163.  A tap of the
+// centre's own normal (one facet of the stone) takes the centre's cosine power again.
+// LAST: the output is the 12-byte image.
+template <int SQ, bool LAST>
+__global__ void __launch_bounds__(256) k_atrous_pass(AtrousConst A, const float4 *__restrict__ src,
+                                                     const float4 *__restrict__ guide, float4 *__restrict__ dst,
+                                                     float *__restrict__ out, int stride) {
+    const uint32_t across = (A.w + 31u) / 32u, tile = blockIdx.x / across;
+    const uint32_t x = (blockIdx.x - tile * across) * 32u + (threadIdx.x & 31u), y = tile * 8u + (threadIdx.x >> 5);
+    if (x >= A.w || y >= A.h) return;
     const float B3[5] = {1.0f / 16.0f, 1.0f / 4.0f, 3.0f / 8.0f, 1.0f / 4.0f, 1.0f / 16.0f};
-    const V3 cc = v3(src[3 * c], src[3 * c + 1], src[3 * c + 2]);
-    const V3 scc = v3(sanitize(cc.x), sanitize(cc.y), sanitize(cc.z));
-    const V3 cn = v3(nn[3 * c], nn[3 * c + 1], nn[3 * c + 2]);
+    const uint64_t c = (uint64_t)y * A.w + x;
+    const float4 c4 = src[c], g4 = guide[c];
+    const V3 scc = v3(sanitize(c4.x), sanitize(c4.y), sanitize(c4.z));
+    const V3 cn = v3(g4.x, g4.y, g4.z);
     const bool cn_zero = cn.x == 0.0f && cn.y == 0.0f && cn.z == 0.0f;
-    const float cdep = sanitize(depth[c]);
-    const int32_t cf = facet[c];
+    const float wn_own =
+        cn_zero ? 1.0f : cos_pow<SQ>(fmaxf(clampf(dot(cn, cn), -1.0f, 1.0f), 0.0f), A.power, A.squarings, A.pow2 != 0);
+    const int32_t cf = __float_as_int(c4.w);
     V3 sum = v3(0.f, 0.f, 0.f);
     float wsum = 0.0f;
 #pragma unroll
     for (int ky = 0; ky < 5; ++ky) {
-        const int64_t sy = y + (int64_t)(ky - 2) * stride;
+        const int64_t sy = (int64_t)y + (ky - 2) * stride;
         if (sy < 0 || sy >= (int64_t)A.h) continue;
+        const float4 *row = src + (uint64_t)sy * A.w, *grow = guide + (uint64_t)sy * A.w;
 #pragma unroll
         for (int kx = 0; kx < 5; ++kx) {
-            const int64_t sx = x + (int64_t)(kx - 2) * stride;
+            const int64_t sx = (int64_t)x + (kx - 2) * stride;
             if (sx < 0 || sx >= (int64_t)A.w) continue;
-            const uint64_t q = (uint64_t)sy * A.w + (uint64_t)sx;
-            if (facet[q] != cf) continue;  // facet_weight 0: the tap is skipped
+            const float4 q4 = row[sx];
+            if (__float_as_int(q4.w) != cf) continue;  // facet_weight 0: the tap is skipped
+            const float4 p4 = grow[sx];
             const float kw = B3[ky] * B3[kx];
-            const V3 qn = v3(nn[3 * q], nn[3 * q + 1], nn[3 * q + 2]);
-            float wn = 1.0f;
-            if (!cn_zero && !(qn.x == 0.0f && qn.y == 0.0f && qn.z == 0.0f))
-                wn = cos_pow(fmaxf(clampf(dot(cn, qn), -1.0f, 1.0f), 0.0f), A.power, A.squarings, A.pow2 != 0);
-            const float wd = expf(fabsf(cdep - sanitize(depth[q])) * A.nisd);
-            const V3 qc = v3(src[3 * q], src[3 * q + 1], src[3 * q + 2]);
-            const V3 dc = v3(scc.x - sanitize(qc.x), scc.y - sanitize(qc.y), scc.z - sanitize(qc.z));
+            const V3 qn = v3(p4.x, p4.y, p4.z);
+            float wn = wn_own;
+            if (qn.x != cn.x || qn.y != cn.y || qn.z != cn.z)
+                wn = (cn_zero || (qn.x == 0.0f && qn.y == 0.0f && qn.z == 0.0f))
+                         ? 1.0f
+                         : cos_pow<SQ>(fmaxf(clampf(dot(cn, qn), -1.0f, 1.0f), 0.0f), A.power, A.squarings, A.pow2 != 0);
+            const float wd = expf(fabsf(g4.w - p4.w) * A.nisd);
+            const V3 qc = v3(q4.x, q4.y, q4.z);
+            V3 sq = qc;
+            if (!(fabsf(qc.x) + fabsf(qc.y) + fabsf(qc.z) < 3.0e38f))  // a component may not be finite
+                sq = v3(sanitize(qc.x), sanitize(qc.y), sanitize(qc.z));
+            const V3 dc = sub(scc, sq);
             const float wc = expf(dot(dc, dc) * A.nits);
             const float wgt = ((kw * wn) * wd) * wc;  // kernel_w * wf * wn * wd * wc with wf = 1
             sum = add(sum, mul(qc, wgt));
             wsum = wsum + wgt;
         }
     }
-    if (wsum > 1.0e-8f) {
-        dst[3 * c + 0] = sum.x / wsum;
-        dst[3 * c + 1] = sum.y / wsum;
-        dst[3 * c + 2] = sum.z / wsum;
+    const V3 r = wsum > 1.0e-8f ? v3(sum.x / wsum, sum.y / wsum, sum.z / wsum) : v3(c4.x, c4.y, c4.z);
+    if (LAST) {
+        out[3 * c + 0] = r.x;
+        out[3 * c + 1] = r.y;
+        out[3 * c + 2] = r.z;
     } else {
-        dst[3 * c + 0] = cc.x;
-        dst[3 * c + 1] = cc.y;
-        dst[3 * c + 2] = cc.z;
+        dst[c] = make_float4(r.x, r.y, r.z, c4.w);
     }
 }
 
@@ -167,20 +198,19 @@ gr_status atrous_device(gr_ctx *ctx, const float *color_in, const float *film, f
     const size_t img = (size_t)n_px * 3 * sizeof(float);
     const float n0 = P.taper_reference_spp > 1.0e-8f ? P.taper_reference_spp : 1.0e-8f;
     const float taper = 1.0f / sqrtf(1.0f + (float)spp / n0);  // taper_strength (:244-250)
-    const unsigned threads = 128;
+    const size_t records = (size_t)n_px * sizeof(float4);
+    const unsigned threads = 256;
     const unsigned blocks = (unsigned)((n_px + threads - 1) / threads);
-    gr_status st = ctx->dn_a.reserve(img);
-    if (st == GR_OK) st = ctx->dn_b.reserve(img);
-    if (st == GR_OK) st = ctx->dn_n.reserve(img);
+    gr_status st = ctx->dn_a.reserve(records);
+    if (st == GR_OK) st = ctx->dn_b.reserve(records);
+    if (st == GR_OK) st = ctx->dn_n.reserve(records);
     if (st != GR_OK) return st;
-    float *a = (float *)ctx->dn_a.ptr, *b = (float *)ctx->dn_b.ptr, *nn = (float *)ctx->dn_n.ptr;
-    grd::k_denoise_prep<<<blocks, threads, 0, s>>>(normal, nn, film ? film : color_in, a, inv_count,
-                                                   film ? 1u : 0u, n_px);
+    float4 *a = (float4 *)ctx->dn_a.ptr, *b = (float4 *)ctx->dn_b.ptr, *guide = (float4 *)ctx->dn_n.ptr;
+    const bool identity = taper < P.taper_identity_epsilon;  // the identity short-circuit: a plain copy
+    grd::k_denoise_prep<<<blocks, threads, 0, s>>>(normal, depth, facet, film ? film : color_in, a, guide,
+                                                   identity ? out : nullptr, inv_count, film ? 1u : 0u, n_px);
     GR_CUDA(cudaGetLastError());
-    if (taper < P.taper_identity_epsilon) {  // the identity short-circuit: a plain copy
-        GR_CUDA(cudaMemcpyAsync(out, a, img, cudaMemcpyDeviceToDevice, s));
-        return GR_OK;
-    }
+    if (identity) return GR_OK;
     const uint32_t passes = P.num_passes < 1 ? 1 : (P.num_passes > 8 ? 8 : P.num_passes);
     const float sce = fmaxf(P.sigma_color * taper, 0.0f);
     const float sd = fmaxf(P.sigma_depth, 1.0e-8f);
@@ -200,15 +230,19 @@ gr_status atrous_device(gr_ctx *ctx, const float *color_in, const float *film, f
             for (uint32_t k = ip; k > 1; k >>= 1) A.squarings++;
         }
     }
+    const unsigned grid = (unsigned)(((w + 31ull) / 32u) * ((h + 7ull) / 8u));
+    const bool six = A.pow2 && A.squarings == 6;
     for (uint32_t pass = 0; pass < passes; ++pass) {
-        float *dst = pass + 1 == passes ? out : b;
-        grd::k_atrous_pass<<<blocks, threads, 0, s>>>(A, a, dst, depth, nn, facet, 1 << pass);
-        GR_CUDA(cudaGetLastError());
-        if (pass + 1 < passes) {
-            float *t = a;
-            a = b;
-            b = t;
+        const int stride = 1 << pass;
+        if (pass + 1 == passes) {
+            if (six) grd::k_atrous_pass<6, true><<<grid, 256, 0, s>>>(A, a, guide, nullptr, out, stride);
+            else grd::k_atrous_pass<0, true><<<grid, 256, 0, s>>>(A, a, guide, nullptr, out, stride);
+        } else {
+            if (six) grd::k_atrous_pass<6, false><<<grid, 256, 0, s>>>(A, a, guide, b, nullptr, stride);
+            else grd::k_atrous_pass<0, false><<<grid, 256, 0, s>>>(A, a, guide, b, nullptr, stride);
+            std::swap(a, b);
         }
+        GR_CUDA(cudaGetLastError());
     }
     return GR_OK;
 }

@@ -2,28 +2,37 @@
 // = evaluate_gem_optical_metrics (crates/gemray/src/color/metrics.rs:1082-1237) for
 // a batch of poses (tilt sweeps, metrics.rs:1262-1289, are batches of poses).
 //
-// k_metric_samples: one thread per (pose, grid cell, slot); slots 0..4 are the five
-//   aperture rays of classify_aperture_sample (metrics.rs:568-676: a d-line trace,
-//   then F- and C-line traces for returned rays), slots 5..9 the five yaw offsets of
-//   cell_temporal_variance (metrics.rs:349-380).  Results land in a per-sample array.
-// k_metric_reduce: one thread per pose folds the samples in the reference's order
-//   (cells ix-major, then aperture order) with the reference's f32 arithmetic, so the
-//   counts are exact and the f32 sums are formed in the same sequence.
+// k_metric_traces: one thread per (pose, trace, cell of the unit disc); traces 0..14 are the
+//   five aperture rays of classify_aperture_sample (metrics.rs:568-676), each at the d, F
+//   and C lines, traces 15..19 the d line at the five yaw offsets of cell_temporal_variance
+//   (metrics.rs:349-380).  Bound by latency (a chain of up to eleven plane scans on a chip
+//   that 16 poses fill to a third), so the three lines of a ray run side by side although
+//   F and C only count where d returns, cells outside the disc get no thread, and the scan
+//   is the transport's branch-free one.
+// k_metric_reduce: one block per pose classifies the samples in parallel and then forms each
+//   of the reference's f32 sums in its order (cells ix-major, then aperture order) in one
+//   thread, the sums side by side in separate warps, so counts are exact and sums are formed
+//   in the same sequence.
+// 16 poses of the 73-plane brilliant: one thread per (pose, cell, ray) with the three lines in
+// turn 746 us and one thread per pose reducing 464 us, 1.22 ms a call; now 0.19 ms a call.
 // Camera bases, the studio rig and the d/F/C indices are host-computed per pose with
 // the reference's f32 libm arithmetic.
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "gemray_cuda.h"
 #include "gr_host.h"
-#include "gr_trace.cuh"
+#include "gr_launch.cuh"
 
 namespace grd {
 
 constexpr int MGRID = 18;
-constexpr int MSLOTS = 10;
+constexpr int MAPS = 5;                    // aperture rays; as many yaw offsets
+constexpr int MTRACES = 3 * MAPS + MAPS;   // per cell
+constexpr int MCELLS_MAX = MGRID * MGRID;
 
 struct PoseConst {
     float fwd[3], right[3], up[3];         // camera_view_basis(cam_yaw, cam_pitch)
@@ -32,10 +41,13 @@ struct PoseConst {
     float nd, nf, nc;                      // indices at 589.3 / 486.1 / 656.3 nm
 };
 
-struct MetricSample {
-    uint32_t cls;   // 0 no hit, 1 entry blocked, 2 windowed, 3 extinct, 4 returned; temporal: 0/1
-    uint32_t fire_valid;
-    float angle_deg, weight;
+// One trace's end: fate 0 entry blocked, 1 leaked, 2 exited upward, 3 absorbed, 4 no hit, 5
+// exited upward and visible (d-line traces).
+struct __align__(16) MetricTrace {
+    uint32_t fate;
+    int32_t facet;
+    uint32_t bounces;
+    float transmittance, exit_cos, dx, dy, dz;
 };
 
 // metrics.rs:118-131
@@ -54,8 +66,8 @@ struct MExit {
 };
 
 // metrics.rs:138-227 (fates: 0 blocked, 1 leaked, 2 exited upward, 3 absorbed)
-__device__ int m_trace_wavelength(V3 entry, V3 in_dir, V3 n_entry, float cos_i, const float4 *planes, uint32_t n,
-                                  float index, MExit &ex) {
+__device__ int m_trace_wavelength(V3 entry, V3 in_dir, V3 n_entry, float cos_i, const Planes &PL, float index,
+                                  MExit &ex) {
     float sin2_t = (1.0f / (index * index)) * fmaf(cos_i, -cos_i, 1.0f);
     if (sin2_t > 1.0f) return 0;
     float cos_t = sqrtf(1.0f - sin2_t);
@@ -67,9 +79,9 @@ __device__ int m_trace_wavelength(V3 entry, V3 in_dir, V3 n_entry, float cos_i, 
     for (uint32_t bounce = 0; bounce < 10; ++bounce) {
         float t = 0.0f;
         int idx = 0;
-        if (!intersect(planes, n, hp, dir, t, idx)) break;
+        if (!intersect_from(PL, true, hp, dir, t, idx)) break;
         V3 np = add(hp, smul(t, dir));
-        V3 n_out = plane_normal(planes, idx);
+        V3 n_out = plane_normal(PL.aos, idx);
         float ct = clampf(dot(dir, n_out), 0.0f, 1.0f);
         float st = sqrtf(fmaxf(fmaf(ct, -ct, 1.0f), 0.0f));
         if (st < sin_crit) {
@@ -110,140 +122,161 @@ __device__ __forceinline__ bool m_visible(V3 d, V3 fwd, const PoseConst &P) {
     return !head && lit;
 }
 
-__device__ __forceinline__ bool cell_uv(int ix, int iz, float &u, float &v) {
+__host__ __device__ __forceinline__ bool cell_uv(int ix, int iz, float &u, float &v) {
     u = fmaf(((float)ix + 0.5f) / (float)MGRID, 2.0f, -1.0f);
     v = fmaf(((float)iz + 0.5f) / (float)MGRID, 2.0f, -1.0f);
     return !(fmaf(v, v, u * u) > 0.70f);
 }
 
-__global__ void k_metric_samples(const PoseConst *__restrict__ poses, uint32_t n_poses, const float4 *__restrict__ gplanes,
-                                 uint32_t n_planes, MetricSample *__restrict__ out) {
+// cells: the disc's cells (ix * MGRID + iz) in the reference's order.
+__global__ void __launch_bounds__(128) k_metric_traces(const PoseConst *__restrict__ poses, uint32_t n_poses,
+                                                       const uint16_t *__restrict__ cells, uint32_t n_cells,
+                                                       const float4 *__restrict__ gplanes, uint32_t n_planes,
+                                                       MetricTrace *__restrict__ out) {
     extern __shared__ float4 s_planes[];
-    for (uint32_t i = threadIdx.x; i < n_planes; i += blockDim.x) s_planes[i] = gplanes[i];
-    __syncthreads();
-    const uint32_t per_pose = MGRID * MGRID * MSLOTS;
+    const Planes PL = stage_plane_set(s_planes, gplanes, n_planes);
     const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (uint64_t)n_poses * per_pose) return;
-    const uint32_t pose = (uint32_t)(gid / per_pose);
-    const uint32_t rem = (uint32_t)(gid % per_pose);
-    const uint32_t cell = rem / MSLOTS, slot = rem % MSLOTS;
-    const int ix = (int)(cell / MGRID), iz = (int)(cell % MGRID);
-    MetricSample r{0u, 0u, 0.0f, 0.0f};
-    float u, v;
-    if (!cell_uv(ix, iz, u, v)) {
-        out[gid] = r;
-        return;
-    }
+    if (gid >= (uint64_t)n_poses * MTRACES * n_cells) return;
+    const uint32_t ray = (uint32_t)(gid / n_cells), cell = cells[gid - (uint64_t)ray * n_cells];
+    const uint32_t pose = ray / MTRACES, trace = ray - pose * MTRACES;
     const PoseConst &P = poses[pose];
-    if (slot < 5) {
+    float u, v;
+    cell_uv((int)(cell / MGRID), (int)(cell % MGRID), u, v);
+    const bool aperture = trace < 3 * MAPS;
+    const uint32_t line = aperture ? trace % 3u : 0u, k = aperture ? trace / 3u : trace - 3u * MAPS;
+    V3 ro, rd, fwd;
+    if (aperture) {
         // classify_aperture_sample (metrics.rs:568-676)
-        const float ap[5][2] = {{0.f, 0.f}, {0.08f, 0.f}, {-0.08f, 0.f}, {0.f, 0.08f}, {0.f, -0.08f}};
-        V3 fwd = ld3(P.fwd), right = ld3(P.right), upv = ld3(P.up);
-        V3 rd = normalize(add(add(fwd, smul(ap[slot][0], right)), smul(ap[slot][1], upv)));
-        V3 ro = add(add(mul(neg(fwd), 2.5f), smul(u * 0.95f, right)), smul(v * 0.95f, upv));
-        float t = 0.0f;
-        int idx = 0;
-        if (intersect(s_planes, n_planes, ro, rd, t, idx)) {
-            V3 hp = add(ro, smul(t, rd));
-            V3 nrm = plane_normal(s_planes, idx);
-            float ci = clampf(dot(neg(rd), nrm), 0.0f, 1.0f);
-            MExit e;
-            int fate = m_trace_wavelength(hp, rd, nrm, ci, s_planes, n_planes, P.nd, e);
-            if (fate == 0) r.cls = 1;
-            else if (fate == 1) r.cls = 2;
-            else if (fate == 3) r.cls = 3;
-            else if (!m_visible(e.dir, fwd, P)) r.cls = 3;
-            else {
-                r.cls = 4;
-                MExit ef, ec;
-                int ff = m_trace_wavelength(hp, rd, nrm, ci, s_planes, n_planes, P.nf, ef);
-                int fc = m_trace_wavelength(hp, rd, nrm, ci, s_planes, n_planes, P.nc, ec);
-                if (ff == 2 && fc == 2 && ef.facet == ec.facet && ef.bounces == ec.bounces) {
-                    float cs = clampf(dot(ef.dir, ec.dir), -1.0f, 1.0f);
-                    r.angle_deg = m_acos(cs) * 57.2957795130823208767981548141051703f;
-                    r.weight = (e.transmittance * ef.transmittance * ec.transmittance) *
-                               (fmaxf(ef.exit_cos, 0.0f) * fmaxf(ec.exit_cos, 0.0f));
-                    r.fire_valid = 1;
-                }
-            }
-        }
+        const float ap[MAPS][2] = {{0.f, 0.f}, {0.08f, 0.f}, {-0.08f, 0.f}, {0.f, 0.08f}, {0.f, -0.08f}};
+        fwd = ld3(P.fwd);
+        const V3 right = ld3(P.right), upv = ld3(P.up);
+        rd = normalize(add(add(fwd, smul(ap[k][0], right)), smul(ap[k][1], upv)));
+        ro = add(add(mul(neg(fwd), 2.5f), smul(u * 0.95f, right)), smul(v * 0.95f, upv));
     } else {
         // cell_returned_at_yaw_offset (metrics.rs:295-330)
-        const uint32_t k = slot - 5;
-        V3 f2 = ld3(P.tf[k]), r2 = ld3(P.tr[k]), u2 = ld3(P.tu[k]);
-        V3 ro = add(add(mul(neg(f2), 2.5f), smul(u * 0.95f, r2)), smul(v * 0.95f, u2));
-        float t = 0.0f;
-        int idx = 0;
-        if (intersect(s_planes, n_planes, ro, f2, t, idx)) {
-            V3 hp = add(ro, smul(t, f2));
-            V3 nrm = plane_normal(s_planes, idx);
-            float ci = clampf(dot(neg(f2), nrm), 0.0f, 1.0f);
-            MExit e;
-            if (m_trace_wavelength(hp, f2, nrm, ci, s_planes, n_planes, P.nd, e) == 2 && m_visible(e.dir, f2, P))
-                r.cls = 1;
+        fwd = rd = ld3(P.tf[k]);
+        ro = add(add(mul(neg(fwd), 2.5f), smul(u * 0.95f, ld3(P.tr[k]))), smul(v * 0.95f, ld3(P.tu[k])));
+    }
+    MetricTrace r{4u, 0, 0u, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    float t = 0.0f;
+    int idx = 0;
+    if (intersect<false>(PL, ro, rd, t, idx)) {
+        const V3 hp = add(ro, smul(t, rd));
+        const V3 nrm = plane_normal(PL.aos, idx);
+        const float ci = clampf(dot(neg(rd), nrm), 0.0f, 1.0f);
+        MExit e;
+        r.fate = (uint32_t)m_trace_wavelength(hp, rd, nrm, ci, PL, line == 0 ? P.nd : (line == 1 ? P.nf : P.nc), e);
+        if (r.fate == 2u) {
+            r.facet = e.facet;
+            r.bounces = e.bounces;
+            r.transmittance = e.transmittance;
+            r.exit_cos = e.exit_cos;
+            r.dx = e.dir.x;
+            r.dy = e.dir.y;
+            r.dz = e.dir.z;
+            if (line == 0 && m_visible(e.dir, fwd, P)) r.fate = 5u;
         }
     }
     out[gid] = r;
 }
 
-// The reference's accumulation order (metrics.rs:1127-1236) per pose.
-__global__ void k_metric_reduce(const MetricSample *__restrict__ in, uint32_t n_poses, gr_metrics_out *__restrict__ out,
-                                uint32_t use_fp64) {
-    const uint32_t pose = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pose >= n_poses) return;
-    const MetricSample *s = in + (size_t)pose * MGRID * MGRID * MSLOTS;
-    uint32_t total = 0, windowed = 0, extinct = 0, returned = 0, cell_count = 0;
-    float fire_sum = 0.f, cf_sum = 0.f, cf_sq = 0.f, tv_sum = 0.f;
-    double fire_d = 0.0, cf_d = 0.0, cf_sq_d = 0.0, tv_d = 0.0;
-    for (int ix = 0; ix < MGRID; ++ix) {
-        for (int iz = 0; iz < MGRID; ++iz) {
-            float u, v;
-            if (!cell_uv(ix, iz, u, v)) continue;
-            const MetricSample *c = s + (size_t)(ix * MGRID + iz) * MSLOTS;
-            uint32_t ct_total = 0, ct_ret = 0;
-            for (int a = 0; a < 5; ++a) {
-                const MetricSample &m = c[a];
-                if (m.cls == 0) continue;
-                total++;
-                ct_total++;
-                if (m.cls == 2) windowed++;
-                else if (m.cls == 3) extinct++;
-                else if (m.cls == 4) {
-                    returned++;
-                    ct_ret++;
-                    if (m.fire_valid) {
-                        fire_sum = fmaf(m.angle_deg, m.weight, fire_sum);
-                        fire_d = fma((double)m.angle_deg, (double)m.weight, fire_d);
-                    }
-                }
-            }
-            if (ct_total > 0) {
-                float frac = (float)ct_ret / (float)ct_total;
-                cf_sum += frac;
-                cf_sq = fmaf(frac, frac, cf_sq);
-                cf_d += (double)frac;
-                cf_sq_d = fma((double)frac, (double)frac, cf_sq_d);
-                cell_count++;
-                uint32_t tr = 0;
-                for (int k = 0; k < 5; ++k) tr += c[5 + k].cls;
-                float tp = (float)tr / 5.0f;
-                tv_sum += fmaf(tp, -tp, tp);
-                tv_d += (double)fmaf(tp, -tp, tp);
+// Sample classes: 0 no hit, 1 entry blocked, 2 windowed, 3 extinct, 4 returned.
+constexpr int MREDUCE_THREADS = 256;
+__global__ void __launch_bounds__(MREDUCE_THREADS) k_metric_reduce(const MetricTrace *__restrict__ in, uint32_t n_cells,
+                                                                   gr_metrics_out *__restrict__ out, uint32_t use_fp64) {
+    __shared__ uint8_t s_cls[MCELLS_MAX * MAPS], s_fire[MCELLS_MAX * MAPS];
+    __shared__ float s_angle[MCELLS_MAX * MAPS], s_weight[MCELLS_MAX * MAPS];
+    __shared__ float s_frac[MCELLS_MAX], s_tv[MCELLS_MAX];
+    __shared__ uint32_t s_count[5];  // samples per class, cells with a hit in [0]
+    __shared__ float s_sum[4];       // fire, cell fraction, its square, temporal variance
+    const MetricTrace *p = in + (size_t)blockIdx.x * MTRACES * n_cells;
+    const uint32_t tid = threadIdx.x;
+    if (tid < 5) s_count[tid] = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < n_cells * MAPS; i += MREDUCE_THREADS) {
+        const uint32_t a = i / n_cells, c = i - a * n_cells, at = c * MAPS + a;  // aperture order within a cell
+        const MetricTrace d = p[(3 * a) * n_cells + c];
+        uint32_t cls = d.fate == 4u ? 0u : (d.fate == 0u ? 1u : (d.fate == 1u ? 2u : (d.fate == 5u ? 4u : 3u)));
+        uint8_t fire = 0;
+        if (cls == 4u) {
+            const MetricTrace f = p[(3 * a + 1) * n_cells + c], g = p[(3 * a + 2) * n_cells + c];
+            if (f.fate == 2u && g.fate == 2u && f.facet == g.facet && f.bounces == g.bounces) {
+                const float cs = clampf(dot(v3(f.dx, f.dy, f.dz), v3(g.dx, g.dy, g.dz)), -1.0f, 1.0f);
+                s_angle[at] = m_acos(cs) * 57.2957795130823208767981548141051703f;
+                s_weight[at] = (d.transmittance * f.transmittance * g.transmittance) *
+                               (fmaxf(f.exit_cos, 0.0f) * fmaxf(g.exit_cos, 0.0f));
+                fire = 1;
             }
         }
+        s_cls[at] = (uint8_t)cls;
+        s_fire[at] = fire;
+        if (cls) atomicAdd(&s_count[cls], 1u);
     }
-    if (use_fp64) {
-        fire_sum = (float)fire_d;
-        cf_sum = (float)cf_d;
-        cf_sq = (float)cf_sq_d;
-        tv_sum = (float)tv_d;
+    __syncthreads();
+    for (uint32_t c = tid; c < n_cells; c += MREDUCE_THREADS) {
+        uint32_t total = 0, ret = 0, tr = 0;
+        for (int a = 0; a < MAPS; ++a) {
+            total += s_cls[c * MAPS + a] != 0;
+            ret += s_cls[c * MAPS + a] == 4;
+            tr += p[(3 * MAPS + a) * n_cells + c].fate == 5u;
+        }
+        s_frac[c] = total ? (float)ret / (float)total : -1.0f;  // -1: no ray of the cell hit
+        const float tp = (float)tr / 5.0f;
+        s_tv[c] = fmaf(tp, -tp, tp);
+        if (total) atomicAdd(&s_count[0], 1u);
     }
+    __syncthreads();
+    // The reference's accumulation order (metrics.rs:1127-1236), one sum per warp.
+    if (tid == 0) {
+        float fire = 0.f;
+        double fire_d = 0.0;
+        for (uint32_t i = 0; i < n_cells * MAPS; ++i) {
+            if (!s_fire[i]) continue;
+            fire = fmaf(s_angle[i], s_weight[i], fire);
+            if (use_fp64) fire_d = fma((double)s_angle[i], (double)s_weight[i], fire_d);
+        }
+        s_sum[0] = use_fp64 ? (float)fire_d : fire;
+    } else if (tid == 32) {
+        float sum = 0.f;
+        double sum_d = 0.0;
+        for (uint32_t c = 0; c < n_cells; ++c) {
+            const float f = s_frac[c];
+            if (f < 0.0f) continue;
+            sum += f;
+            if (use_fp64) sum_d += (double)f;
+        }
+        s_sum[1] = use_fp64 ? (float)sum_d : sum;
+    } else if (tid == 64) {
+        float sq = 0.f;
+        double sq_d = 0.0;
+        for (uint32_t c = 0; c < n_cells; ++c) {
+            const float f = s_frac[c];
+            if (f < 0.0f) continue;
+            sq = fmaf(f, f, sq);
+            if (use_fp64) sq_d = fma((double)f, (double)f, sq_d);
+        }
+        s_sum[2] = use_fp64 ? (float)sq_d : sq;
+    } else if (tid == 96) {
+        float tv = 0.f;
+        double tv_d = 0.0;
+        for (uint32_t c = 0; c < n_cells; ++c) {
+            if (s_frac[c] < 0.0f) continue;
+            tv += s_tv[c];
+            if (use_fp64) tv_d += (double)s_tv[c];
+        }
+        s_sum[3] = use_fp64 ? (float)tv_d : tv;
+    }
+    __syncthreads();
+    if (tid != 0) return;
+    const uint32_t windowed = s_count[2], extinct = s_count[3], returned = s_count[4], cell_count = s_count[0];
+    const uint32_t total = s_count[1] + windowed + extinct + returned;
+    const float cf_sum = s_sum[1], cf_sq = s_sum[2], tv_sum = s_sum[3];
     const float nt = (float)(total > 1 ? total : 1);
     gr_metrics_out o;
     o.windowing_pct = clampf((float)windowed / nt * 100.0f, 0.0f, 100.0f);
     o.extinction_pct = clampf((float)extinct / nt * 100.0f, 0.0f, 100.0f);
     o.brilliance_pct = clampf((float)returned / nt * 100.0f, 0.0f, 100.0f);
-    o.fire_index = fmaxf(fire_sum / nt * 275.0f, 0.1f);
+    o.fire_index = fmaxf(s_sum[0] / nt * 275.0f, 0.1f);
     float spatial = 0.0f;
     if (cell_count > 0) {
         float mean = cf_sum / (float)cell_count;
@@ -255,7 +288,7 @@ __global__ void k_metric_reduce(const MetricSample *__restrict__ in, uint32_t n_
     }
     float temporal = cell_count > 0 ? clampf((tv_sum / (float)cell_count) / 0.24f * 100.0f, 0.0f, 100.0f) : 0.0f;
     o.scintillation_pct = clampf(fmaf(0.4f, temporal, 0.6f * spatial), 0.0f, 100.0f);
-    out[pose] = o;
+    out[blockIdx.x] = o;
 }
 
 }  // namespace grd
@@ -304,17 +337,19 @@ namespace grh {
 void studio_rig(float yaw, float pitch, float key[3], float fill[3], float ring[16][3]);
 
 namespace {
+// The inputs (poses, cell list, planes) first, in one upload; then traces and results.
 struct MetricsLayout {
-    size_t pose_bytes, plane_bytes, sample_bytes, out_bytes;
-    size_t total() const { return pose_bytes + plane_bytes + sample_bytes + out_bytes; }
+    size_t cell_off, plane_off, in_bytes, trace_bytes, out_bytes;
+    size_t total() const { return in_bytes + trace_bytes + out_bytes; }
 };
+size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
 MetricsLayout metrics_layout(uint32_t n_planes, uint32_t n_poses) {
-    const size_t per_pose = (size_t)grd::MGRID * grd::MGRID * grd::MSLOTS;
     MetricsLayout L;
-    L.pose_bytes = ((n_poses * sizeof(grd::PoseConst)) + 255) & ~(size_t)255;
-    L.plane_bytes = (((size_t)(n_planes ? n_planes : 1) * sizeof(float4)) + 255) & ~(size_t)255;
-    L.sample_bytes = ((n_poses * per_pose * sizeof(grd::MetricSample)) + 255) & ~(size_t)255;
-    L.out_bytes = n_poses * sizeof(gr_metrics_out);
+    L.cell_off = up256((size_t)n_poses * sizeof(grd::PoseConst));
+    L.plane_off = L.cell_off + up256(grd::MCELLS_MAX * sizeof(uint16_t));
+    L.in_bytes = L.plane_off + up256((size_t)(n_planes ? n_planes : 1) * sizeof(float4));
+    L.trace_bytes = up256((size_t)n_poses * grd::MTRACES * grd::MCELLS_MAX * sizeof(grd::MetricTrace));
+    L.out_bytes = (size_t)n_poses * sizeof(gr_metrics_out);
     return L;
 }
 }  // namespace
@@ -323,7 +358,19 @@ size_t metrics_scratch_bytes(uint32_t n_planes, uint32_t n_poses) { return metri
 
 gr_status metrics_device(const gr_plane *planes, uint32_t n_planes, const gr_material *m, const gr_pose *poses,
                          uint32_t n_poses, gr_metrics_out *out, uint32_t flags, cudaStream_t stream, DeviceBuffer &scratch) {
-    std::vector<grd::PoseConst> pc(n_poses);
+    const MetricsLayout L = metrics_layout(n_planes, n_poses);
+    gr_status st = scratch.reserve(L.total());
+    if (st != GR_OK) return st;
+    std::vector<char> staged(L.in_bytes);
+    grd::PoseConst *pc = (grd::PoseConst *)staged.data();
+    uint16_t *cells = (uint16_t *)(staged.data() + L.cell_off);
+    uint32_t n_cells = 0;
+    for (int ix = 0; ix < grd::MGRID; ++ix)
+        for (int iz = 0; iz < grd::MGRID; ++iz) {
+            float u, v;
+            if (grd::cell_uv(ix, iz, u, v)) cells[n_cells++] = (uint16_t)(ix * grd::MGRID + iz);
+        }
+    if (n_planes) std::memcpy(staged.data() + L.plane_off, planes, n_planes * sizeof(gr_plane));
     const float nd = fmaxf(host_dispersion(m->dispersion, 589.3f), 1.1f);
     const float nf = fmaxf(host_dispersion(m->dispersion, 486.1f), 1.001f);
     const float nc = fmaxf(host_dispersion(m->dispersion, 656.3f), 1.001f);
@@ -341,29 +388,19 @@ gr_status metrics_device(const gr_plane *planes, uint32_t n_planes, const gr_mat
         P.nf = nf;
         P.nc = nc;
     }
-    const size_t per_pose = (size_t)grd::MGRID * grd::MGRID * grd::MSLOTS;
-    const MetricsLayout L = metrics_layout(n_planes, n_poses);
-    const size_t pose_bytes = L.pose_bytes, plane_bytes = L.plane_bytes, sample_bytes = L.sample_bytes,
-                 out_bytes = L.out_bytes;
-    gr_status st = scratch.reserve(L.total());
-    if (st != GR_OK) return st;
     char *base = (char *)scratch.ptr;
-    grd::PoseConst *d_pose = (grd::PoseConst *)base;
-    float4 *d_planes = (float4 *)(base + pose_bytes);
-    grd::MetricSample *d_samp = (grd::MetricSample *)(base + pose_bytes + plane_bytes);
-    gr_metrics_out *d_out = (gr_metrics_out *)(base + pose_bytes + plane_bytes + sample_bytes);
-    if (cudaMemcpyAsync(d_pose, pc.data(), n_poses * sizeof(grd::PoseConst), cudaMemcpyHostToDevice, stream) != cudaSuccess)
-        return GR_ECUDA;
-    if (n_planes && cudaMemcpyAsync(d_planes, planes, n_planes * sizeof(gr_plane), cudaMemcpyHostToDevice, stream) != cudaSuccess)
-        return GR_ECUDA;
-    const uint64_t threads = (uint64_t)n_poses * per_pose;
+    grd::MetricTrace *d_traces = (grd::MetricTrace *)(base + L.in_bytes);
+    gr_metrics_out *d_out = (gr_metrics_out *)(base + L.in_bytes + L.trace_bytes);
+    if (cudaMemcpyAsync(base, staged.data(), L.in_bytes, cudaMemcpyHostToDevice, stream) != cudaSuccess) return GR_ECUDA;
+    const uint64_t threads = (uint64_t)n_poses * grd::MTRACES * n_cells;
     const unsigned T = 128;
-    grd::k_metric_samples<<<(unsigned)((threads + T - 1) / T), T, n_planes * sizeof(float4), stream>>>(
-        d_pose, n_poses, d_planes, n_planes, d_samp);
-    grd::k_metric_reduce<<<(n_poses + 63) / 64, 64, 0, stream>>>(d_samp, n_poses, d_out,
-                                                                 (flags & GR_METRICS_FP64_SUMS) ? 1u : 0u);
+    grd::k_metric_traces<<<(unsigned)((threads + T - 1) / T), T, grd::planes_smem_bytes(n_planes), stream>>>(
+        (const grd::PoseConst *)base, n_poses, (const uint16_t *)(base + L.cell_off), n_cells,
+        (const float4 *)(base + L.plane_off), n_planes, d_traces);
+    grd::k_metric_reduce<<<n_poses, grd::MREDUCE_THREADS, 0, stream>>>(d_traces, n_cells, d_out,
+                                                                       (flags & GR_METRICS_FP64_SUMS) ? 1u : 0u);
     if (cudaGetLastError() != cudaSuccess) return GR_ECUDA;
-    if (cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess) return GR_ECUDA;
+    if (cudaMemcpyAsync(out, d_out, L.out_bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess) return GR_ECUDA;
     if (cudaStreamSynchronize(stream) != cudaSuccess) return GR_ECUDA;
     return GR_OK;
 }

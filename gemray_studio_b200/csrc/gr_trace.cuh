@@ -284,12 +284,9 @@ __device__ __forceinline__ uint32_t channel_tables(Path &P, const SceneConst &S,
     return any ? F_ABSORBING : 0u;
 }
 
-// Convex clip against planes staged in shared memory (intersect.rs:93-132,
-// simd/slab.rs:101-152).  Returns false on a miss.
-//
-// The reference divides t = -side/denom for every plane, but a plane's t only
-// matters if it can raise the running near maximum (denom < 0) or lower the running
-// far minimum (denom > 0).  q' = (-side) * rcp.approx(denom) is within 2^-21 relative
+// The convex clip (intersect.rs:93-132, simd/slab.rs:101-152).  The reference divides
+// t = -side/denom for every plane, but a plane's t only matters if it can raise the running
+// near maximum (denom < 0) or lower the running far minimum (denom > 0).  q' = (-side) * rcp.approx(denom) is within 2^-21 relative
 // of the exact quotient q; if q' + |q'| 2^-19 < t_near then q < t_near, so the
 // correctly rounded fl(q) <= t_near and the plane cannot update (rounding is
 // monotone) -- likewise for the far side.  Only the remaining planes take the IEEE
@@ -298,48 +295,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
-}
-
-__device__ __forceinline__ bool intersect(const float4 *__restrict__ planes, uint32_t n, V3 o, V3 d, float &t_hit,
-                                          int &idx_hit) {
-    float t_near = -1e30f, t_far = 1e30f;
-    int near_idx = -1, far_idx = -1;
-    bool outside = false;
-#pragma unroll 2
-    for (uint32_t i = 0; i < n; ++i) {
-        float4 p = planes[i];
-        float denom = (p.x * d.x + p.y * d.y) + p.z * d.z;
-        float side = p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z);
-        if (fabsf(denom) > 1e-7f) {
-            const float num = -side;
-            const float qa = num * rcp_approx(denom);
-            const float margin = fabsf(qa) * 1.9073486e-6f;  // 2^-19
-            if (denom < 0.0f) {
-                if (!(qa + margin < t_near)) {
-                    float t = num / denom;
-                    if (t > t_near) { t_near = t; near_idx = (int)i; }
-                }
-            } else if (!(qa - margin > t_far)) {
-                float t = num / denom;
-                if (t < t_far) { t_far = t; far_idx = (int)i; }
-            }
-        } else if (side > 0.0f) {
-            outside = true;
-            break;
-        }
-    }
-    if (outside || t_near > t_far) return false;
-    if (t_near > 1e-4f) {
-        t_hit = t_near;
-        idx_hit = near_idx;
-        return true;
-    }
-    if (t_far > 1e-4f) {
-        t_hit = t_far;
-        idx_hit = far_idx;
-        return true;
-    }
-    return false;
 }
 
 // ---------------------------------------------------------------------------------

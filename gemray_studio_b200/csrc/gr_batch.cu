@@ -228,14 +228,14 @@ gr_status launch_plan(const Plan &P, const grd::SceneSlot *slots, const grd::Bat
         GR_CUDA(cudaMemsetAsync(counts, 0, (size_t)L.seg_count * sizeof(unsigned int), s));
         if (L.extras) {
             grd::launch_batch_grids<true, grd::K_ANY, GR_TRACE_MIN_BLOCKS>(slots, segs + L.seg_first, L.seg_count, L.chunk, park,
-                                                                           counts, L.blocks, L.park_blocks, smem, s);
+                                                                           counts, L.blocks, L.park_blocks, smem, grd::camera_smem_bytes(L.max_planes), s);
         } else if (L.K >= 0) {
             const gr_status st = grh::launch_batch_class(L.K, slots, segs + L.seg_first, L.seg_count, L.chunk, park, counts,
-                                                         L.blocks, L.park_blocks, smem, s);
+                                                         L.blocks, L.park_blocks, smem, grd::camera_smem_bytes(L.max_planes), s);
             if (st != GR_OK) return st;
         } else {
             grd::launch_batch_grids<false, grd::K_ANY, GR_TRACE_MIN_BLOCKS>(slots, segs + L.seg_first, L.seg_count, L.chunk, park,
-                                                                            counts, L.blocks, L.park_blocks, smem, s);
+                                                                            counts, L.blocks, L.park_blocks, smem, grd::camera_smem_bytes(L.max_planes), s);
         }
         const unsigned T = 256;
         grd::k_fold_batch<<<(unsigned)((L.warps * 32 + T - 1) / T), T, 0, s>>>(segs + L.seg_first, L.seg_count);

@@ -73,12 +73,13 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     __syncthreads();
     const SceneConst &S = s_slot.S;
     const SceneBuffers &B = s_slot.B;
-    const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
+    Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
+    stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), ld3(S.cam_o));
     const LaunchRange R = G.R;
     const uint64_t first = (uint64_t)(blockIdx.x - G.block_begin) * chunk;
     float *xyz = G.xyz;
     Path P;
-    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K>(
+    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K, true>(
         P, S, B, PL, PoolRange{first, min(first + chunk, R.n_tuples)}, G.stage_cap,
         ParkOut{park + G.park_off, G.park_cap, counts + s_seg},
         [&](Path &q, uint64_t t) {
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     const Path *from = park + G.park_off;
     float *xyz = G.xyz;
     Path P;
-    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K>(
+    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K, false>(
         P, S, B, PL, PoolRange{j0, min(j0 + blockDim.x, (uint64_t)n)}, 0xFFFFFFFFu, ParkOut{nullptr, 0, nullptr},
         [&](Path &q, uint64_t i) { copy_record<record_rows<EXTRAS, K>()>(q, from[i]); },
         [&](const Path &q) { store_sample(xyz, q, path_finish<1, false, K, EXTRAS>(q, S, B)); });
@@ -121,9 +122,9 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
 // One batched launch's two trace grids for scene class K at MB blocks per SM.
 template <bool EXTRAS, int K, int MB>
 void launch_batch_grids(const SceneSlot *slots, const BatchSegment *segs, uint32_t n_segs, uint32_t chunk, Path *park,
-                        unsigned int *counts, uint64_t blocks, uint64_t park_blocks, size_t smem, cudaStream_t s) {
+                        unsigned int *counts, uint64_t blocks, uint64_t park_blocks, size_t smem, size_t cam_smem, cudaStream_t s) {
     constexpr int T = pool_threads<EXTRAS, K>();
-    k_trace_batch<EXTRAS, K, MB><<<(unsigned)blocks, T, smem, s>>>(slots, segs, n_segs, chunk, park, counts);
+    k_trace_batch<EXTRAS, K, MB><<<(unsigned)blocks, T, smem + cam_smem, s>>>(slots, segs, n_segs, chunk, park, counts);
     k_trace_batch_cont<EXTRAS, K, MB><<<(unsigned)park_blocks, T, smem, s>>>(slots, segs, n_segs, park, counts);
 }
 

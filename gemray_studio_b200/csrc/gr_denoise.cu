@@ -24,36 +24,43 @@ using grh::fail;
 
 namespace grd {
 
+// A grid of resident blocks strides over the pixels, so each block stages the planes and the
+// camera's table once.
 __global__ void __launch_bounds__(128) k_guide_pass(SceneConst S, const float4 *__restrict__ gplanes,
                                                     float *__restrict__ depth, float *__restrict__ normal,
                                                     int32_t *__restrict__ facet) {
     extern __shared__ float4 s_planes[];
-    const Planes PL = stage_plane_set(s_planes, gplanes, S.n_planes);
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint64_t)S.width * S.height) return;
-    const uint32_t x = (uint32_t)(i % S.width), y = (uint32_t)(i / S.width);
-    const float aspect = S.width_f / S.height_f;
-    const float u = (((float)x + 0.0f) / S.width_f - 0.5f) * 2.0f * aspect * S.fov_tan;
-    const float v = (0.5f - ((float)y + 0.0f) / S.height_f) * 2.0f * S.fov_tan;
-    const V3 dir = normalize(add(add(ld3(S.cam_f), mul(ld3(S.cam_r), u)), mul(ld3(S.cam_u), v)));
-    float t = 0.0f;
-    int idx = -1;
-    float d = 1.0e6f;
-    V3 n = v3(0.f, 0.f, 0.f);
-    int32_t f = -1;
-    if (intersect<false>(PL, ld3(S.cam_o), dir, t, idx)) {
-        d = t;
-        if (idx >= 0) {  // an empty plane set hits at t = 1e30 with the zero normal, facet 0
-            const float4 p = PL.aos[idx];
-            n = v3(p.x, p.y, p.z);
+    Planes PL = stage_plane_set(s_planes, gplanes, S.n_planes);
+    const V3 o = ld3(S.cam_o);
+    stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), o);
+    const uint64_t n_px = (uint64_t)S.width * S.height, step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_px; i += step) {
+        const uint32_t y = (uint32_t)(i / S.width), x = (uint32_t)(i - (uint64_t)y * S.width);
+        const float aspect = S.width_f / S.height_f;
+        const float u = (((float)x + 0.0f) / S.width_f - 0.5f) * 2.0f * aspect * S.fov_tan;
+        const float v = (0.5f - ((float)y + 0.0f) / S.height_f) * 2.0f * S.fov_tan;
+        const V3 dir = normalize(add(add(ld3(S.cam_f), mul(ld3(S.cam_r), u)), mul(ld3(S.cam_u), v)));
+        float t = 0.0f;
+        int idx = -1;
+        float d = 1.0e6f;
+        V3 n = v3(0.f, 0.f, 0.f);
+        int32_t f = -1;
+        int r = intersect_camera(PL, dir, o, t, idx);
+        if (r == SCAN_UNDECIDED) r = intersect<false>(PL, o, dir, t, idx) ? SCAN_HIT : SCAN_MISS;
+        if (r == SCAN_HIT) {
+            d = t;
+            if (idx >= 0) {  // an empty plane set hits at t = 1e30 with the zero normal, facet 0
+                const float4 p = PL.aos[idx];
+                n = v3(p.x, p.y, p.z);
+            }
+            f = idx >= 0 ? idx : 0;
         }
-        f = idx >= 0 ? idx : 0;
+        depth[i] = d;
+        normal[3 * i + 0] = n.x;
+        normal[3 * i + 1] = n.y;
+        normal[3 * i + 2] = n.z;
+        facet[i] = f;
     }
-    depth[i] = d;
-    normal[3 * i + 0] = n.x;
-    normal[3 * i + 1] = n.y;
-    normal[3 * i + 2] = n.z;
-    facet[i] = f;
 }
 
 __device__ __forceinline__ float sanitize(float v) { return isfinite(v) ? v : 0.0f; }
@@ -274,8 +281,10 @@ gr_status guide_device(gr_ctx *ctx, const gr_scene *sc, float *depth, float *nor
         GR_CUDA(cudaMemcpyAsync(ctx->dn_planes.ptr, sc->planes, sc->n_planes * sizeof(gr_plane), cudaMemcpyHostToDevice,
                                 ctx->stream));
     const unsigned threads = 128;
-    grd::k_guide_pass<<<(unsigned)((n_px + threads - 1) / threads), threads, grd::planes_smem_bytes(S.n_planes),
-                        ctx->stream>>>(S, (const float4 *)ctx->dn_planes.ptr, depth, normal, facet);
+    const uint64_t resident = (uint64_t)(ctx->sm_count > 0 ? ctx->sm_count : 1) * 12u, need = (n_px + threads - 1) / threads;
+    grd::k_guide_pass<<<(unsigned)(need < resident ? need : resident), threads,
+                        grd::planes_smem_bytes(S.n_planes) + grd::camera_smem_bytes(S.n_planes), ctx->stream>>>(
+        S, (const float4 *)ctx->dn_planes.ptr, depth, normal, facet);
     GR_CUDA(cudaGetLastError());
     // the host planes are copied from pageable memory: wait before the caller may free them
     GR_CUDA(cudaStreamSynchronize(ctx->stream));

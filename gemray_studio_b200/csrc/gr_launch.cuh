@@ -40,6 +40,61 @@ __device__ __forceinline__ Planes stage_plane_set(float4 *sp, const float4 *__re
     return Planes{sp, pairs, n};
 }
 
+// The camera's table of the staged planes (intersect_camera) at ct, camera_smem_bytes(n):
+// built by the first warp, one plane per lane; the whole block calls.
+__device__ __forceinline__ void stage_camera_table(Planes &PL, float4 *ct, V3 o) {
+    if (threadIdx.x < 32u) {
+        const uint32_t lane = threadIdx.x;
+        auto side_of = [&](uint32_t i) {
+            const float4 p = PL.aos[i];
+            return p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z);
+        };
+        uint32_t n1 = 0, bad = 0;
+        float min1 = 3.0e38f, min2 = 3.0e38f;
+        for (uint32_t b = 0; b < PL.n; b += 32u) {
+            const bool on = b + lane < PL.n;
+            const float s = on ? side_of(b + lane) : -1.0f;
+            bad |= __ballot_sync(0xffffffffu, on && !(fabsf(s) >= 1e-6f && fabsf(s) < 1e15f));
+            n1 += __popc(__ballot_sync(0xffffffffu, on && s > 0.0f));
+            if (on && s > 0.0f) min1 = fminf(min1, s);
+            else if (on) min2 = fminf(min2, -s);
+        }
+        for (int k = 16; k; k >>= 1) {
+            min1 = fminf(min1, __shfl_xor_sync(0xffffffffu, min1, k));
+            min2 = fminf(min2, __shfl_xor_sync(0xffffffffu, min2, k));
+        }
+        const uint32_t n2 = PL.n - n1, p1 = (n1 + 1u) / 2u, p2 = p1 + (n2 + 1u) / 2u;
+        if (lane == 0)
+            ct[0] = make_float4(__uint_as_float(bad ? 0u : p1), __uint_as_float(p2), 1.001e-7f / min1, 1.001e-7f / min2);
+        float *f = reinterpret_cast<float *>(ct + 1);
+        auto put = [&](uint32_t pair, uint32_t half, float4 p, float rs, float bias, uint32_t i) {
+            float *e = f + 12u * pair + half;
+            e[0] = p.x;
+            e[2] = p.y;
+            e[4] = p.z;
+            e[6] = rs;
+            e[8] = bias;
+            e[10] = __uint_as_float(i);
+        };
+        uint32_t c1 = 0;
+        for (uint32_t b = 0; b < PL.n && !bad; b += 32u) {
+            const uint32_t i = b + lane;
+            const bool on = i < PL.n;
+            const float s = on ? side_of(i) : -1.0f;
+            const uint32_t m = __ballot_sync(0xffffffffu, on && s > 0.0f), below = (1u << lane) - 1u;
+            const uint32_t r1 = c1 + __popc(m & below), r2 = i - r1;
+            if (on && s > 0.0f) put(r1 / 2u, r1 & 1u, PL.aos[i], -1.0f / s, 0.0f, i);
+            else if (on) put(p1 + r2 / 2u, r2 & 1u, PL.aos[i], -1.0f / s, 0.0f, i);
+            c1 += __popc(m);
+        }
+        const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (lane == 0 && !bad && (n1 & 1u)) put(p1 - 1u, 1u, none, 0.0f, 3.0e38f, 0u);
+        if (lane == 0 && !bad && (n2 & 1u)) put(p2 - 1u, 1u, none, 0.0f, -3.0e38f, 0u);
+    }
+    PL.cam = ct;
+    __syncthreads();
+}
+
 __device__ __forceinline__ void tuple_coords(const LaunchRange &R, uint64_t t, uint32_t &pixel, uint32_t &sample) {
     uint32_t local_pixel = (uint32_t)(t / R.spp);
     uint32_t s = (uint32_t)(t - (uint64_t)local_pixel * R.spp);

@@ -134,10 +134,10 @@ template <int T, uint32_t ROWS> __device__ __forceinline__ void pack_block(Path 
 // made DRAIN_CAPS * `cap` bounces are parked in `out` while it has slots.  Called by the whole block of
 // T threads; every barrier is reached by all of them.
 // Packing without a refill (the drain) waits until a quarter of the warps would be freed: a
-// swap costs about a tenth of a bounce.  Refilling at three quarters instead of half a block
+// swap costs about a tenth of a bounce.  CAM: the planes carry the camera's table.  Refilling at three quarters instead of half a block
 // measured 43.3 against 40.5 ms on the brilliant and 48.6 against 43.8 on the emerald: more
 // swaps, and finishes and starts in smaller groups.
-template <int T, bool EXTRAS, int K, class Supply, class Start, class Store>
+template <int T, bool EXTRAS, int K, bool CAM, class Supply, class Start, class Store>
 __device__ __forceinline__ void run_pool(Path &P, const SceneConst &S, const SceneBuffers &B, const Planes &PL,
                                          Supply supply, uint32_t cap, const ParkOut &out, Start start, Store store) {
     __shared__ uint64_t s_base;
@@ -189,7 +189,7 @@ __device__ __forceinline__ void run_pool(Path &P, const SceneConst &S, const Sce
         uint32_t ev = EV_DONE;
         float t_hit = 0.0f;
         int fidx = 0;
-        const bool hit = go && step_scan<NoCounters, false>(P, PL, t_hit, fidx, nc);
+        const bool hit = go && step_scan<NoCounters, false, CAM>(P, PL, t_hit, fidx, nc);
         __syncthreads();
         if (hit) ev = step_facet<GR_STEP_UNROLL, NoCounters, false, EXTRAS, K>(P, S, B, PL, t_hit, fidx, E, nc);
         __syncthreads();

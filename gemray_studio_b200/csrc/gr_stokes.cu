@@ -28,9 +28,10 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K_ANY>(), pool_blocks(MB,
     k_trace_stokes(SceneConst S, SceneBuffers B, LaunchRange R, float *__restrict__ xyz, float4 *__restrict__ iquv,
                    unsigned long long *work) {
     extern __shared__ float4 s_planes[];
-    const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
+    Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
+    stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), ld3(S.cam_o));
     Path P;
-    run_pool<pool_threads<EXTRAS, K_ANY>(), EXTRAS, K_ANY>(
+    run_pool<pool_threads<EXTRAS, K_ANY>(), EXTRAS, K_ANY, true>(
         P, S, B, PL, PoolQueue{work, R.n_tuples}, 0xFFFFFFFFu, ParkOut{nullptr, 0, nullptr},
         [&](Path &q, uint64_t t) {
             uint32_t pixel, sample;
@@ -113,7 +114,7 @@ gr_status gr_accumulate_stokes(gr_ctx *ctx, const gr_scene *sc, uint32_t sample_
     if (st != GR_OK) return st;
     float *txyz = (float *)ctx->xyz.ptr;
     float4 *tiquv = (float4 *)((char *)ctx->xyz.ptr + toff);
-    const size_t smem = grd::planes_smem_bytes(S.n_planes);
+    const size_t smem = grd::planes_smem_bytes(S.n_planes) + grd::camera_smem_bytes(S.n_planes);
     st = ctx->counter.reserve(64);
     if (st != GR_OK) return st;
     for (uint64_t first = 0; first < n_pixels; first += chunk_pixels) {

@@ -322,6 +322,7 @@ struct Planes {
     const float4 *aos;    // n x (n.xyz, d)
     const float4 *pairs;  // ceil(n / 2) x 2 float4, interleaved as above
     uint32_t n;
+    const float4 *cam = nullptr;  // the camera's table (stage_camera_table), if staged
 };
 
 __host__ __device__ constexpr size_t planes_smem_bytes(uint32_t n) {
@@ -349,6 +350,12 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b, f32x2 one) {
     f32x2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(one), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
 
@@ -410,11 +417,23 @@ __device__ __forceinline__ bool scan_plane(float denom, float side, int i, float
 //
 // Why: the general scan's updates and divisions are branches, and among the lanes of a
 // warp some lane takes them at nearly every plane, so the warp pays for them 73 times a
-// bounce; this scan issues 14 instructions per plane whatever the lanes do.
+// bounce; this scan issues 13 instructions per plane whatever the lanes do (not unrolled: by
+// 2 the brilliant at 32 spp took 39.1 ms against 37.6).
 constexpr int SCAN_MISS = 0, SCAN_HIT = 1, SCAN_UNDECIDED = 2;
 constexpr uint32_t SCAN_INDEX_MASK = GR_MAX_PLANES - 1u;
 static_assert((GR_MAX_PLANES & (GR_MAX_PLANES - 1)) == 0 && GR_MAX_PLANES <= 512, "the index fits the key's low 9 bits");
 
+// sm_100's three-input minimum and maximum (a NaN among them is passed over, as in fminf).
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 __device__ __forceinline__ float scan_key(float v, uint32_t i) {
     return __uint_as_float((__float_as_uint(v) & ~SCAN_INDEX_MASK) | i);
 }
@@ -423,6 +442,10 @@ __device__ __forceinline__ float scan_key(float v, uint32_t i) {
 #define GR_SCAN_UNROLL 1
 #endif
 constexpr int SCAN_UNROLL = GR_SCAN_UNROLL;
+#ifndef GR_CAM_UNROLL
+#define GR_CAM_UNROLL 1
+#endif
+constexpr int CAM_UNROLL = GR_CAM_UNROLL;
 __device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, float &t_hit, int &idx_hit) {
     const f32x2 dx = pk2(d.x, d.x), dy = pk2(d.y, d.y), dz = pk2(d.z, d.z);
     const f32x2 ox = pk2(o.x, o.x), oy = pk2(o.y, o.y), oz = pk2(o.z, o.z);
@@ -437,10 +460,10 @@ __device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, fl
         float den0, den1, sid0, sid1;
         upk2(add2(add2(mul2(nx, dx), mul2(ny, dy), one), mul2(nz, dz), one), den0, den1);
         upk2(add2(add2(add2(mul2(nx, ox), mul2(ny, oy), one), mul2(nz, oz), one), pk2(b.z, b.w), one), sid0, sid1);
-        side_max = fmaxf(side_max, fmaxf(sid0, sid1));
+        side_max = max3(side_max, sid0, sid1);
         const float k0 = scan_key(den0 * rcp_approx(sid0), i), k1 = scan_key(den1 * rcp_approx(sid1), i + 1u);
         const float lo = fminf(k0, k1), hi = fmaxf(k0, k1);
-        second = fminf(fminf(second, hi), fmaxf(best, lo));
+        second = min3(second, hi, fmaxf(best, lo));
         best = fminf(best, lo);
     }
     if (!(side_max < -1e-30f) || !(best < -1e-20f) || !(second > best * (1.0f - 4.8828125e-4f))) return SCAN_UNDECIDED;
@@ -452,6 +475,67 @@ __device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, fl
     t_hit = (-side) / denom;
     idx_hit = idx;
     return t_hit > 1e-4f ? SCAN_HIT : SCAN_MISS;
+}
+
+// The scan of the rays that start at the camera.  Their origin is the launch's, so every
+// plane's side is too: the block splits the planes once into those the camera is beyond
+// (side > 0, entered where the ray hits) and those it is not (side < 0, left), with rs =
+// -1 / side, and a ray needs only denom: u = denom * rs = 1 / t orders both lists.  The entry
+// facet has the least u of the first list, the exit the greatest of the second.  Sides of
+// zero or without a clear sign turn the table off.
+// Table: a header (pairs of the first list, of both, bound of u below which a plane of the
+// first / second list may count as parallel), then per pair {nx0, nx1, ny0, ny1}, {nz0, nz1,
+// rs0, rs1}, {bias0, bias1, index0, index1}; the bias takes an odd list's padding out.
+__host__ __device__ constexpr size_t camera_smem_bytes(uint32_t n) { return (size_t)(1u + 3u * (n / 2u + 1u)) * 16u; }
+
+// As intersect_inside: keys with the index in 9 bits, exact quotient for the winner alone, and
+// SCAN_UNDECIDED within 2^-11 of a tie or of a parallel plane.
+// Every primary ray took the general scan; with the table the brilliant at 32 spp went from
+// 39.0 to 37.7 ms (16 blocks), the emerald from 38.8 to 38.0 (12), 64 batched stones from 28.3
+// to 27.3, guide pass + filter + tone map of 1920x1080 from 1.143 to 1.120 ms.
+__device__ __forceinline__ int intersect_camera(const Planes &PL, V3 d, V3 o, float &t_hit, int &idx_hit) {
+    const float4 head = PL.cam[0];
+    const uint32_t p1 = __float_as_uint(head.x), p2 = __float_as_uint(head.y);
+    if (p1 == 0u) return SCAN_UNDECIDED;
+    const f32x2 dx = pk2(d.x, d.x), dy = pk2(d.y, d.y), dz = pk2(d.z, d.z);
+    const float unit = __uint_as_float(0x3f800000u | (PL.n >> 16));  // 1.0f, as in intersect_inside
+    const f32x2 one = pk2(unit, unit);
+    float near = 3.0e38f, near2 = 3.0e38f, far = -3.0e38f;
+    const float4 *q = PL.cam + 1, *const q1 = q + 3 * p1, *const q2 = q + 3 * p2;
+    auto keys = [&](const float4 *e, float &k0, float &k1) {
+        const float4 a = e[0], b = e[1], c = e[2];
+        const f32x2 den =
+            add2(add2(mul2(pk2(a.x, a.y), dx), mul2(pk2(a.z, a.w), dy), one), mul2(pk2(b.x, b.y), dz), one);
+        float u0, u1;
+        upk2(fma2(den, pk2(b.z, b.w), pk2(c.x, c.y)), u0, u1);
+        k0 = scan_key(u0, __float_as_uint(c.z));
+        k1 = scan_key(u1, __float_as_uint(c.w));
+    };
+#pragma unroll CAM_UNROLL
+    for (; q < q1; q += 3) {
+        float k0, k1;
+        keys(q, k0, k1);
+        const float lo = fminf(k0, k1), hi = fmaxf(k0, k1);
+        near2 = min3(near2, hi, fmaxf(near, lo));
+        near = fminf(near, lo);
+    }
+#pragma unroll CAM_UNROLL
+    for (; q < q2; q += 3) {
+        float k0, k1;
+        keys(q, k0, k1);
+        far = max3(far, k0, k1);
+    }
+    if (near < -head.z) return SCAN_MISS;  // a plane the origin is beyond, and the ray leaves
+    if (!(near > head.z) || !(far > head.w)) return SCAN_UNDECIDED;
+    if (near < far * (1.0f - 4.8828125e-4f)) return SCAN_MISS;  // leaves before it has entered
+    if (!(near > far * (1.0f + 4.8828125e-4f)) || !(near2 > near * (1.0f + 4.8828125e-4f))) return SCAN_UNDECIDED;
+    const int idx = (int)(__float_as_uint(near) & SCAN_INDEX_MASK);
+    const float4 p = PL.aos[idx];
+    const float denom = (p.x * d.x + p.y * d.y) + p.z * d.z;
+    const float side = p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z);
+    t_hit = (-side) / denom;
+    idx_hit = idx;
+    return denom < -1e-7f && t_hit > 1e-4f && t_hit < 1e29f ? SCAN_HIT : SCAN_UNDECIDED;
 }
 
 // The reference clip (intersect.rs:93-132) in FP64, t rounded back to f32: the
@@ -776,12 +860,17 @@ __device__ __forceinline__ float theta_c(V3 kk, V3 normal, float cos_i, float on
 //
 // step_scan: false on an escape (F_ESCAPED set, F_ALIVE cleared; accumulate_miss_radiance,
 // transport.rs:67-90, runs in path_finish).
-template <class CT, bool R = false>
+// CAM: the planes carry the camera's table; a path that has made no bounce starts there.
+template <class CT, bool R = false, bool CAM = false>
 __device__ __forceinline__ bool step_scan(Path &P, const Planes &PL, float &t_hit, int &fidx, CT &ct) {
     const uint32_t bits = state_bits(P);
     const V3 o = xyz(P.o_hero), d = xyz(P.d_seed);
     tally(ct, C_BOUNCES);
-    if (!intersect_from<R>(PL, (bits & F_INSIDE) != 0, o, d, t_hit, fidx)) {
+    int r = SCAN_UNDECIDED;
+    if (CAM && bits_bounce(bits) == 0) r = intersect_camera(PL, d, o, t_hit, fidx);
+    else if (!R && (bits & F_INSIDE)) r = intersect_inside(PL, o, d, t_hit, fidx);
+    if (r == SCAN_UNDECIDED) r = intersect<R>(PL, o, d, t_hit, fidx) ? SCAN_HIT : SCAN_MISS;
+    if (r == SCAN_MISS) {
         tally(ct, C_ESCAPES);
         note_end(ct, bits_bounce(bits), GR_TERM_ESCAPED);
         set_state_bits(P, (bits | F_ESCAPED) & ~F_ALIVE);

@@ -57,9 +57,10 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     k_trace_pool(SceneConst S, SceneBuffers B, LaunchRange R, float *__restrict__ xyz, unsigned long long *work,
                  ParkOut out, uint32_t bounce_cap) {
     extern __shared__ float4 s_planes[];
-    const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
+    Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
+    stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), ld3(S.cam_o));
     Path P;
-    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K>(
+    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K, true>(
         P, S, B, PL, PoolQueue{work, R.n_tuples}, bounce_cap, out,
         [&](Path &q, uint64_t t) {
             uint32_t pixel, sample;
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     extern __shared__ float4 s_planes[];
     const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
     Path P;
-    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K>(
+    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K, false>(
         P, S, B, PL, PoolQueue{work, n}, bounce_cap, out,
         [&](Path &q, uint64_t i) { copy_record<record_rows<EXTRAS, K>()>(q, park_in[i]); },
         [&](const Path &q) { store_sample(xyz, q, path_finish<1, false, K, EXTRAS>(q, S, B)); });
@@ -105,7 +106,7 @@ void launch_pool(const SceneConst &S, const SceneBuffers &B, const LaunchRange &
     const uint64_t resident = (uint64_t)L.sm_count * pool_blocks(MB, T), need = (R.n_tuples + T - 1) / T;
     const unsigned grid = (unsigned)(need < resident ? need : resident);
     const ParkOut out1{L.park1, L.cap1, L.counts}, out2{L.park2, L.cap2, L.counts + 1}, none{nullptr, 0, nullptr};
-    k_trace_pool<EXTRAS, K, MB><<<grid, T, smem, stream>>>(S, B, R, xyz, L.work, out1, L.cap_first);
+    k_trace_pool<EXTRAS, K, MB><<<grid, T, smem + camera_smem_bytes(S.n_planes), stream>>>(S, B, R, xyz, L.work, out1, L.cap_first);
     k_trace_resume<EXTRAS, K, MB><<<grid, T, smem, stream>>>(S, B, L.park1, L.cap1, L.counts, L.cap_second, L.work + 1,
                                                              out2, xyz);
     k_trace_resume<EXTRAS, K, MB><<<grid, T, smem, stream>>>(S, B, L.park2, L.cap2, L.counts + 1, 0xFFFFFFFFu, L.work + 2,

@@ -52,6 +52,28 @@ def test_pool_is_the_plain_kernel(pair, kind, size):
     assert np.array_equal(films[0].view(np.uint32), films[1].view(np.uint32))
 
 
+@pytest.mark.parametrize("kind", ["clear", "general", "extras"])
+@pytest.mark.parametrize("planes", [1, 2, 511, 512])
+def test_pool_with_few_and_most_planes(pair, kind, planes):
+    """The camera's table: one-sided plane sets (rays that never leave), odd lists, the plane
+    limit (the most shared memory), and a camera inside the stone or on one of its planes."""
+    for cam in (S.camera(0.4, 0.5, 4.0, 26.0), S.camera(0.4, 0.5, 0.1, 40.0), S.camera(0.0, np.pi / 2, 1.0, 40.0)):
+        films = []
+        for r in pair:
+            sc = _scene(kind, 24, 17, 12)
+            far = np.tile(np.asarray([[0.6, 0.8, 0.0, -50.0]], np.float32), (512, 1))
+            sc.planes = np.concatenate([sc.planes, far])[:planes]
+            if planes < 3:
+                sc.planes[0] = (0.0, 1.0, 0.0, -1.0)  # the last camera sits on this plane
+            sc.cam = cam
+            if sc.finishes is not None:
+                sc.finishes = np.zeros(len(sc.planes), np.uint32)
+            acc = np.zeros((24 * 17, 3), np.float32)
+            r.accumulate(sc, 0, 9, acc)
+            films.append(acc)
+        assert np.array_equal(films[0].view(np.uint32), films[1].view(np.uint32))
+
+
 @pytest.mark.parametrize("kind", ["clear", "general"])
 def test_paths_past_the_drain_limit(pair, kind):
     """Depth 4096 in a uniform environment: the longest paths are parked and resumed."""

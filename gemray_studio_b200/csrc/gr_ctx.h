@@ -240,6 +240,7 @@ struct StagedLaunch {
     uint32_t cap_first, cap_second;
     uint32_t blocks;  // kScheduleBlocks entry, 0 = builtin_schedule_blocks
     int sm_count;
+    bool alone;       // the first launch only, nothing parked (small launches under AUTO)
 };
 // The plain kernel (st == NULL) or the three staged launches of scene class K
 // (gr_single_clear.cu / gr_single_general.cu).

@@ -479,6 +479,7 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
                        float *xyz, cudaStream_t stream, int mode, grh::DeviceBuffer *park_buf, StageCaps caps) {
     if (caps.first == 0) caps = StageCaps{GR_STAGE_CAP, GR_STAGE_CAP2};
     if (R.n_tuples == 0) return GR_OK;
+    const int asked = mode;
     mode = scene_kernel(mode, S, R.n_tuples);
     size_t smem = grd::planes_smem_bytes(S.n_planes);
     const bool extras = grd::needs_extras(S);
@@ -495,10 +496,18 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
     }
     const int K = scene_class(S);
     const bool clear = K >= 0 && (K & grd::K_CLEAR);
+    // Launches under AUTO's staged size that the pool runs better alone: its blocks fetch
+    // together, which pays sooner the longer the class's code.  Measured (plain / pool, us):
+    // birefringent 262,144 tuples 561 / 555, 409,600 782 / 620; frosted biaxial 65,536 929 /
+    // 973, 147,456 1272 / 1163, 409,600 2370 / 1456; clear 409,600 784 / 858 (never).
+    const bool pool_alone = mode == GR_KERNEL_PLAIN && asked != GR_KERNEL_PLAIN && S.max_bounces > 0 &&
+                            (extras ? R.n_tuples >= (1u << 17) : (!clear && R.n_tuples >= (1u << 18)));
+    if (pool_alone) mode = GR_KERNEL_STAGED;
     if (mode == GR_KERNEL_PLAIN || S.max_bounces == 0) {
         if (extras) {
-            grd::k_trace_plain<grd::NoCounters, false, true><<<(unsigned)plain_blocks, grd::TRACE_THREADS, smem, stream>>>(
-                S, B, R, xyz, nullptr);
+            const uint32_t lanes = grd::plain_lanes(R.n_tuples, false);
+            grd::k_trace_plain<grd::NoCounters, false, true>
+                <<<grd::plain_blocks(R.n_tuples, lanes), grd::TRACE_THREADS, smem, stream>>>(S, B, R, xyz, nullptr, lanes);
             GR_CUDA(cudaGetLastError());
             return GR_OK;
         }
@@ -514,9 +523,9 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
         return launch_single_clear(K, S, B, R, xyz, stream, nullptr, (unsigned int *)pk.ptr + 2, ctx->sm_count);
     }
     if (mode == GR_KERNEL_STAGED) {
-        const uint64_t slots = staged_park_slots(R.n_tuples, ctx->sm_count);
+        const uint64_t slots = pool_alone ? 0 : staged_park_slots(R.n_tuples, ctx->sm_count);
         grh::DeviceBuffer &pk = park_buf ? *park_buf : ctx->park;
-        gr_status st = pk.reserve(staged_park_bytes(R.n_tuples, ctx->sm_count));
+        gr_status st = pk.reserve(pool_alone ? kParkHeader : staged_park_bytes(R.n_tuples, ctx->sm_count));
         if (st != GR_OK) return st;
         GR_CUDA(cudaMemsetAsync(pk.ptr, 0, kParkHeader, stream));
         StagedLaunch sl;
@@ -529,6 +538,7 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
         sl.cap_second = caps.second;
         sl.blocks = caps.blocks;
         sl.sm_count = ctx->sm_count > 0 ? ctx->sm_count : 1;
+        sl.alone = pool_alone;
         if (!extras)
             return clear ? launch_single_clear(K, S, B, R, xyz, stream, &sl)
                          : launch_single_general(K, S, B, R, xyz, stream, &sl);

@@ -11,7 +11,7 @@ namespace grh {
 
 inline grd::PoolLaunch pool_launch(const StagedLaunch &st) {
     return grd::PoolLaunch{st.park1, st.park2, (uint32_t)st.cap1, (uint32_t)st.cap2, st.counts, st.work,
-                           st.cap_first, st.cap_second, st.sm_count};
+                           st.cap_first, st.cap_second, st.sm_count, st.alone};
 }
 
 // The three pooled launches at MB blocks per SM.
@@ -31,9 +31,9 @@ gr_status launch_single_k(const SceneConst &S, const grd::SceneBuffers &B, const
                           cudaStream_t stream, const StagedLaunch *st) {
     if (!st) {
         const size_t smem = grd::planes_smem_bytes(S.n_planes);
-        const unsigned blocks = (unsigned)((R.n_tuples + grd::TRACE_THREADS - 1) / grd::TRACE_THREADS);
+        const uint32_t lanes = grd::plain_lanes(R.n_tuples, (K & grd::K_CLEAR) != 0);
         grd::k_trace_plain<grd::NoCounters, false, false, K, GR_TRACE_MIN_BLOCKS>
-            <<<blocks, grd::TRACE_THREADS, smem, stream>>>(S, B, R, xyz, nullptr);
+            <<<grd::plain_blocks(R.n_tuples, lanes), grd::TRACE_THREADS, smem, stream>>>(S, B, R, xyz, nullptr, lanes);
         GR_CUDA(cudaGetLastError());
         return GR_OK;
     }

@@ -9,7 +9,7 @@
 
 namespace grd {
 
-// Plain kernel: one thread traces one tuple start to finish -- the reference
+// Plain kernel: one thread traces one tuple start to finish, `lanes` tuples per warp -- the reference
 // kernel's launch shape (one invocation per (pixel, sample), spectral_transport.wgsl:
 // 672-691).  The Counters variant tallies events for the FLOP model; RESOLVE is the
 // GR_FLAG_FP64_RESOLVE variant (FP64 re-solve of ambiguous exits and TIR decisions);
@@ -18,10 +18,13 @@ namespace grd {
 template <class CT, bool RESOLVE = false, bool EXTRAS = false, int K = K_ANY, int MB = GR_TRACE_MIN_BLOCKS>
 __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_plain(SceneConst S, SceneBuffers B, LaunchRange R,
                                                                float *__restrict__ xyz,
-                                                               unsigned long long *__restrict__ tallies) {
+                                                               unsigned long long *__restrict__ tallies,
+                                                               uint32_t lanes = 32) {
     extern __shared__ float4 s_planes[];
     const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint64_t t = R.n_tuples;
+    if ((threadIdx.x & 31u) < lanes)
+        t = ((uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u) * lanes + (threadIdx.x & 31u);
     CT ct;
     if constexpr (sizeof(CT) == sizeof(Counters)) {
         for (int i = 0; i < C_COUNT; ++i) ((Counters &)ct).c[i] = 0;
@@ -45,6 +48,24 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_plain(SceneConst S,
             if (lane == 0 && v) atomicAdd(tallies + i, v);
         }
     }
+}
+
+// Paths per warp of a plain launch.  A launch that leaves the chip idle waits for its longest
+// path, and a warp runs the branches and channels of all its paths in turn: fewer paths per
+// warp shorten that chain while each of the 4 x 148 schedulers has few warps.  Measured on
+// the 73-plane brilliant, studio, depth 32 (us at 32 / 16 / 8 / 4 paths per warp): 4,608
+// tuples 339 / 296 / 278 / 253 clear, 211 / 185 / 169 / 155 birefringent, 725 / 717 / 647 /
+// 643 biaxial; 16,384 tuples 348 / 309 / 295 / 317, 259 / 244 / 257 / 282, 771 / 738 / 751 /
+// 902; 36,864 tuples 405 / 348 / 351 / 412, 263 / 304 / 325 / 445, 780 / 863 / 1023 / 1280.
+inline uint32_t plain_lanes(uint64_t n_tuples, bool clear) {
+    const uint64_t per_lane = 4 * 4 * 148;  // four warps on every scheduler
+    if (n_tuples <= 4 * per_lane) return 4;
+    if (clear) return n_tuples <= 8 * per_lane ? 8 : (n_tuples <= 16 * per_lane ? 16 : 32);
+    return n_tuples <= 8 * per_lane ? 16 : 32;
+}
+inline unsigned plain_blocks(uint64_t n_tuples, uint32_t lanes) {
+    const uint64_t per = (uint64_t)lanes * (TRACE_THREADS / 32);
+    return (unsigned)((n_tuples + per - 1) / per);
 }
 
 // Pooled kernels (the scheme and run_pool are in gr_stage.cuh), three launches per trace:
@@ -97,6 +118,7 @@ struct PoolLaunch {
     unsigned long long *work;
     uint32_t cap_first, cap_second;
     int sm_count;
+    bool alone;  // the first launch only, nothing parked
 };
 template <bool EXTRAS, int K, int MB>
 void launch_pool(const SceneConst &S, const SceneBuffers &B, const LaunchRange &R, float *xyz, cudaStream_t stream,
@@ -106,7 +128,9 @@ void launch_pool(const SceneConst &S, const SceneBuffers &B, const LaunchRange &
     const uint64_t resident = (uint64_t)L.sm_count * pool_blocks(MB, T), need = (R.n_tuples + T - 1) / T;
     const unsigned grid = (unsigned)(need < resident ? need : resident);
     const ParkOut out1{L.park1, L.cap1, L.counts}, out2{L.park2, L.cap2, L.counts + 1}, none{nullptr, 0, nullptr};
-    k_trace_pool<EXTRAS, K, MB><<<grid, T, smem + camera_smem_bytes(S.n_planes), stream>>>(S, B, R, xyz, L.work, out1, L.cap_first);
+    k_trace_pool<EXTRAS, K, MB><<<grid, T, smem + camera_smem_bytes(S.n_planes), stream>>>(
+        S, B, R, xyz, L.work, L.alone ? none : out1, L.cap_first);
+    if (L.alone) return;
     k_trace_resume<EXTRAS, K, MB><<<grid, T, smem, stream>>>(S, B, L.park1, L.cap1, L.counts, L.cap_second, L.work + 1,
                                                              out2, xyz);
     k_trace_resume<EXTRAS, K, MB><<<grid, T, smem, stream>>>(S, B, L.park2, L.cap2, L.counts + 1, 0xFFFFFFFFu, L.work + 2,

@@ -53,6 +53,22 @@ def test_pool_is_the_plain_kernel(pair, kind, size):
 
 
 @pytest.mark.parametrize("kind", ["clear", "general", "extras"])
+@pytest.mark.parametrize("size", [(1, 1, 3), (37, 64, 4), (37, 65, 4), (74, 65, 4), (148, 65, 4), (128, 64, 16), (128, 128, 16)])
+def test_auto_small_launches_are_the_pool(pair, engine_lib, kind, size):
+    """AUTO's choices below its staged size: 4, 8, 16 or 32 paths per warp (2,368 tuples a
+    path), the pool alone from 2^17 (extension kernels) and 2^18 tuples (general classes)."""
+    w, h, spp = size
+    auto = GpuFrameRenderer()
+    films = []
+    for r in (auto, pair[0]):
+        acc = np.full((w * h, 3), 0.25, np.float32)
+        r.accumulate(_scene(kind, w, h, 24), 5, spp, acc)
+        films.append(acc)
+    auto.close()
+    assert np.array_equal(films[0].view(np.uint32), films[1].view(np.uint32))
+
+
+@pytest.mark.parametrize("kind", ["clear", "general", "extras"])
 @pytest.mark.parametrize("planes", [1, 2, 511, 512])
 def test_pool_with_few_and_most_planes(pair, kind, planes):
     """The camera's table: one-sided plane sets (rays that never leave), odd lists, the plane

@@ -80,13 +80,15 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     extern __shared__ float4 s_planes[];
     Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
     stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), ld3(S.cam_o));
+    __shared__ HeroOrder H;
+    if (R.spp >= HERO_MIN_SPP) hero_order(H, R);
     Path P;
     run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K, true>(
         P, S, B, PL, PoolQueue{work, R.n_tuples}, bounce_cap, out,
         [&](Path &q, uint64_t t) {
-            uint32_t pixel, sample;
-            tuple_coords(R, t, pixel, sample);
-            path_init<K>(q, S, pixel, sample, (uint32_t)t);
+            uint32_t px, s;
+            hero_coords(R, H, t, px, s);
+            path_init<K>(q, S, R.first_pixel + px, R.sample_offset + s, px * R.spp + s);
         },
         [&](const Path &q) { store_sample(xyz, q, path_finish<1, false, K, EXTRAS>(q, S, B)); });
 }

@@ -17,7 +17,7 @@ Prints ONE JSON line (rank 0):
   e2e     the same metric through the reference-facing C-ABI call gr_accumulate with
           host buffers (host->device upload of scene + film and the film readback
           inside the timed region);
-  roofline  FP32 bound of the transport (k_trace_stage1 + k_trace_stage2): algorithmic
+  roofline  FP32 bound of the transport (k_trace_pool + k_trace_resume): algorithmic
           flops from the event-tallied FLOP model / its event-timed duration, against
           the FP32 FMA throughput measured on this device;
   cpu_baseline  the C++ restatement of the reference CPU tracer on this host's cores;
@@ -277,7 +277,7 @@ def run_reference(args):
     }), flush=True)
 
 
-TRANSPORT_LABELS = {"staged": "k_trace_stage1 + k_trace_stage2 x2 (staged transport)", "plain": "k_trace_plain",
+TRANSPORT_LABELS = {"staged": "k_trace_pool + k_trace_resume x2 (pooled transport)", "plain": "k_trace_plain",
                     "sorted": "k_trace_sorted (block-sorted transport)"}
 
 

@@ -11,9 +11,9 @@
 // and the per-pixel fold order are those of the single-scene kernels: every film is
 // bit-identical to rendering its item alone with gr_render_resident.
 //
-// Launches are staged like the single-scene renders (gr_stage.cuh): k_trace_batch runs
-// paths up to the stage cap and parks the survivors in their segment's park region,
-// k_trace_batch_cont finishes them, one block per 128 parked paths of one segment.
+// Launches are pooled like the single-scene renders (gr_stage.cuh): a k_trace_batch block runs
+// its pool over up to kBatchFills blocks' worth of one segment's tuples; k_trace_batch_cont
+// finishes the few paths that outlive its drain, one block's worth of one segment per block.
 //
 // With GR_BATCH_GRAPH the launch sequence is captured once as a CUDA graph and
 // replayed whenever the same batch shape recurs (same scenes, films, spp, frame sizes
@@ -74,7 +74,7 @@ struct Plan {
 
 // Park slots per launch: 1/16 of its tuples (paths alive after the stage cap are a few
 // percent on the stones measured), at most 4 GiB of records; a segment whose region
-// fills up finishes the rest of its paths in stage 1.
+// fills up finishes the rest of its paths in its own pools.
 constexpr uint64_t kBatchParkLimit = (4ull << 30) / sizeof(grd::Path);
 
 // A trace block's run of tuples: as many blocks' worth as the launch has device fills (1,024

@@ -27,20 +27,17 @@ gr_status fail(gr_status st, const char *fmt, ...);
         if (e_ != cudaSuccess) return grh::fail(GR_ECUDA, "%s failed: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
-// Bounce caps of the staged kernels' first two stages ({0, 0} = the built-in pair) and
-// the resident blocks per SM their register allocation targets (0 =
-// builtin_schedule_blocks): a staged schedule.
+// A staged schedule: the bounce caps of the pooled trace's first two launches ({0, 0} = the
+// built-in pair; they act on paths that outlive eight times their value while a block drains)
+// and the resident blocks per SM their register allocation targets, in blocks of 128 threads
+// (0 = builtin_schedule_blocks).
 struct StageCaps {
     uint32_t first = 0, second = 0;
     uint32_t blocks = 0;
 };
-// Blocks-per-SM targets the staged single-scene kernels are built for: register
-// budgets of 56 / 48 / 40 / 32 per thread on 128-thread blocks (a target of 11 compiles
-// to the same 40 registers as 12, 13-15 to the same 32 as 16).  Measured on B200, ms
-// per frame at 9 / 10 / 12 / 16 blocks: the c2 brilliant (caps 12 / 20) 554.8 / 542.7 /
-// 531.0 / 513.4, the c3 emerald (caps 8 / 16) 2019.6 / 1970.1 / 1937.1 / 1904.4 -- the
-// latency of the scalar physics code is hidden better by more warps than it costs in
-// spilled values.
+// Blocks-per-SM targets the pooled single-scene kernels are built for, in blocks of 128
+// threads: whole blocks of 256 (4, 5, 6, 8 per SM at 64, 48, 40, 32 registers) or of 512 (2,
+// 2, 3, 4 at 64, 64, 40, 32).
 constexpr int kScheduleBlockCount = 4;
 constexpr uint32_t kScheduleBlocks[kScheduleBlockCount] = {9, 10, 12, 16};
 // The blocks per SM of a pooled launch whose schedule is still open: 16 for the clear
@@ -50,9 +47,7 @@ constexpr uint32_t kScheduleBlocks[kScheduleBlockCount] = {9, 10, 12, 16};
 constexpr uint32_t builtin_schedule_blocks(int scene_class) {
     return scene_class >= 0 && (scene_class & 2 /* grd::K_CLEAR */) ? 16u : 12u;
 }
-// Stage-cap pairs a stone chooses between: the pair measured best on the c2 brilliant
-// (long, TIR-trapped diamond paths), the one measured best on the c3 emerald (n ~ 1.6,
-// shorter paths; 3.9% faster there) and a longer pair for longer paths still.
+// Cap pairs a stone chooses between (of little effect below depths of 64).
 constexpr int kCapPairCount = 3;
 constexpr uint32_t kCapPairs[kCapPairCount][2] = {{12, 20}, {8, 16}, {16, 28}};
 // Candidate schedules: cap pair p at blocks b is candidate p * kScheduleBlockCount + b.
@@ -133,7 +128,7 @@ struct gr_ctx {
     int sm_count = 0;
     grh::DeviceBuffer xyz, film, planes, map, ext, counter, rgba, metrics;
     int kernel_mode = GR_KERNEL_AUTO;
-    // staged kernels' park buffer (count word, then parked path records)
+    // pooled kernels' park buffer (a header of counters, then parked path records)
     grh::DeviceBuffer park;
     // Optional per-launch timing of the trace and fold kernels (CUDA events on the
     // launch stream); read back by gr_timing_read.

@@ -1,7 +1,8 @@
 // gr_sorted.cuh -- the block-sorted transport kernel for clear isotropic stones
 // (GR_KERNEL_SORTED).
 //
-// In the plain and staged kernels a thread owns one path from start to end, so a warp
+// In the plain kernel, and in the one-path-per-thread stages that were the default when this
+// form was measured, a thread owns one path from start to end, so a warp
 // runs every event kind its 32 paths take at a bounce (reflect and refract, one after
 // the other with part of the warp masked off) and waits for its longest path.  Here a
 // block of SORT_THREADS threads owns SORT_THREADS path slots in shared memory, and any
@@ -26,7 +27,8 @@
 // are only half busy (barrier stalls 3.2 cycles per issue): 11.1 ms against the staged
 // kernels' 9.1 ms.  A variant with one compaction and one combined event + refill +
 // intersection phase per round (three barriers) was slower still (12.5 ms): its rounds
-// last as long as their slowest warp.  The staged kernels stay the default.
+// last as long as their slowest warp.  The default is the pooled form (gr_stage.cuh),
+// which keeps records in local memory, packs instead of sorting and has four barriers a bounce.
 //
 // Layout: a slot is the PATH_CLEAR_BYTES of Path a clear isotropic stone uses followed
 // by its EVENT_ISO_BYTES of Event, padded to SORT_SLOT_BYTES = 304 B: 76 words, so

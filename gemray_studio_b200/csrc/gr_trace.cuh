@@ -3,20 +3,23 @@
 // stages over a path record:
 //
 //   path_init    sampler draws, camera ray, per-sample wavelength cache
-//   step_hit     one intersection; on a hit: Stokes frame rotation, interior
-//                Beer-Lambert absorption, refraction geometry and the hero's event
-//                decision (TIR / partial reflect / refract) -> Event
+//   step_scan    one intersection
+//   step_facet   on a hit: Stokes frame rotation, interior Beer-Lambert absorption,
+//                refraction geometry and the hero's event decision (TIR / partial
+//                reflect / refract) -> Event (step_hit: step_scan and step_facet)
 //   step_reflect the TIR and partial-reflect channel updates (one loop: a TIR event
 //                is the reflect update with scale factor exactly 1.0)
 //   step_refract the refract channel updates (chromatic termination, walk-off)
+//   step_leave   ends a path that leaves through the facet it met (pooled kernels)
 //   path_finish  escape radiance, spectral MIS, CIE integration, white balance
 //
-// The plain and staged kernels run the stages back to back in one thread; the sorted
-// kernel (gr_sorted.cuh) keeps records in shared-memory slots and lets any thread of
+// The plain kernel runs the stages back to back in one thread; the pooled kernels
+// (gr_stage.cuh) run each stage for the whole block and move records between threads; the
+// sorted kernel (gr_sorted.cuh) keeps records in shared-memory slots and lets any thread of
 // the block run any slot's next stage, grouped by event kind.  `Path` is a record of
-// float4 rows: in the plain kernel it lives in the thread's local memory, in the
-// sorted kernel in shared memory, in the staged kernels' park buffers in global
-// memory -- the same code serves all of them.
+// float4 rows: in the plain and pooled kernels it lives in the thread's local memory, in
+// the sorted kernel in shared memory, in the park buffers in global memory -- the same code
+// serves all of them.
 #pragma once
 
 #include <cstddef>
@@ -27,23 +30,9 @@ namespace grd {
 
 constexpr int NCH = 8;
 
-// Unroll factors of the per-channel loops on the bounce path (code size vs. issue).
-#ifndef GR_ROT_UNROLL
-#define GR_ROT_UNROLL 8
-#endif
-#ifndef GR_RR_UNROLL
-#define GR_RR_UNROLL 4  // measured on the c2 frame: 4 beats 8 / 2 / 1 by 1-3% (code layout)
-#endif
-// The rotation loop of the general (absorbing or birefringent) scene classes: measured
-// at 16 blocks per SM, unrolled by 2 / 4 / 8, the c3 emerald 585.5 / 580.7 / 563.6 M
-// path-samples/s and the c4 random stones one at a time at full size 571 / 583 / 577 M;
-// the clear brilliant wants 8 (1,032.6 against 1,017.2 at 4 and 1,009.6 at 2).  The best
-// factor follows the kernel's code layout; 4 is the best for both general workloads.
-#ifndef GR_ROT_UNROLL_GENERAL
-#define GR_ROT_UNROLL_GENERAL 4
-#endif
-constexpr int ROT_UNROLL = GR_ROT_UNROLL;
-constexpr int RR_UNROLL = GR_RR_UNROLL;
+// Unroll factor of the per-channel loops that take every channel (the extension kernels and
+// the event counters; the default kernels walk their live channels, rolled).
+constexpr int ALL_UNROLL = 4;
 
 // Per-path record (352 B).  Flag bits live in k_state.w's integer view.
 struct __align__(16) Path {
@@ -91,10 +80,6 @@ constexpr int K_ISO = 1;        // S.anisotropic == 0 (and not biaxial)
 constexpr int K_CLEAR = 2;      // S.absorbing == 0: no absorption data at all
 constexpr int K_ENV_SHIFT = 2;  // bits 2-3: 0 = the environment kind at run time, else GR_ENV_* + 1
 __host__ __device__ constexpr int k_env(uint32_t env) { return (int)(env + 1) << K_ENV_SHIFT; }
-// The rotation loop's unroll factor in the kernels of scene class K.
-__host__ __device__ constexpr int rot_unroll(int K) {
-    return (K != K_ANY && !(K & K_CLEAR)) ? GR_ROT_UNROLL_GENERAL : GR_ROT_UNROLL;
-}
 template <int K> __device__ __forceinline__ bool aniso_k(const SceneConst &S) {
     return (K & K_ISO) ? false : (S.anisotropic != 0);
 }
@@ -717,7 +702,7 @@ __device__ __forceinline__ void advance_bounce(Path &P, const SceneConst &S, CT 
     const uint32_t bounce = bits_bounce(bits);
     if (bounce > 4) {
         float mx = 0.0f;
-#pragma unroll RR_UNROLL
+#pragma unroll ALL_UNROLL
         for (int k = 0; k < NCH; ++k) mx = fmaxf(mx, fmaxf(P.st[k].x, 0.0f));
         const float q = clampf(mx, 0.05f, 1.0f);
         if (rng_draw(p_seed(P), bounce, RUSSIAN_ROULETTE_STREAM) > q) {
@@ -726,7 +711,7 @@ __device__ __forceinline__ void advance_bounce(Path &P, const SceneConst &S, CT 
             return;
         }
         const float iq = 1.0f / q;
-#pragma unroll RR_UNROLL
+#pragma unroll ALL_UNROLL
         for (int k = 0; k < NCH; ++k) {
             const float4 s4 = P.st[k];
             P.st[k] = make_float4(s4.x * iq, s4.y * iq, s4.z * iq, s4.w * iq);
@@ -914,7 +899,7 @@ __device__ __forceinline__ uint32_t step_facet(Path &P, const SceneConst &S, con
     if (dot(cur_plane, cur_plane) > 1e-6f && dot(prev, prev) > 1e-6f) {
         float psi = signed_psi(prev, cur_plane, kk);
         float2 sc = m_sincos(2.0f * psi);
-        each_channel<live_only<CT, X>, rot_unroll(K)>(live, [&](int k) {
+        each_channel<live_only<CT, X>, ALL_UNROLL>(live, [&](int k) {
             float4 s = P.st[k];
             const Stokes in{s.x, s.y, s.z, s.w};
             const Stokes r = live_only<CT, X> ? rotate_finite<(K & K_CLEAR) != 0>(in, sc.y, sc.x)
@@ -1039,7 +1024,7 @@ __device__ __forceinline__ void step_post(Path &P, const SceneConst &S, V3 hp, V
         tally(ct, C_ROULETTE);
         const uint32_t live = live_channels<CT, X>(bits);
         float mx = 0.0f;
-        each_channel<live_only<CT, X>, RR_UNROLL>(live, [&](int k) { mx = fmaxf(mx, fmaxf(P.st[k].x, 0.0f)); });
+        each_channel<live_only<CT, X>, ALL_UNROLL>(live, [&](int k) { mx = fmaxf(mx, fmaxf(P.st[k].x, 0.0f)); });
         float q = clampf(mx, 0.05f, 1.0f);
         if (rng_draw(seed, bounce, RUSSIAN_ROULETTE_STREAM) > q) {
             tally(ct, C_ROULETTE_KILLS);
@@ -1048,7 +1033,7 @@ __device__ __forceinline__ void step_post(Path &P, const SceneConst &S, V3 hp, V
             return;
         }
         const float iq = 1.0f / q;
-        each_channel<live_only<CT, X>, RR_UNROLL>(live, [&](int k) {
+        each_channel<live_only<CT, X>, ALL_UNROLL>(live, [&](int k) {
             float4 s = P.st[k];
             P.st[k] = make_float4(s.x * iq, s.y * iq, s.z * iq, s.w * iq);
         });

@@ -18,7 +18,7 @@
  *     (crates/gemray/src/geometry/plane.rs:6-9, renderer/buffers.rs:148-165,236-299),
  *     so a Rust caller can pass `bytemuck::bytes_of(&GpuGemMaterial::encode(m))`.
  *   - Calls on one context are serialised by its mutex, and its device scratch (the
- *     per-tuple XYZ chunk, the staged kernels' park records, batch tables) is reused
+ *     per-tuple XYZ chunk, the pooled kernels' park records, batch tables) is reused
  *     call after call in stream order.  Work a caller queues on its own streams must
  *     therefore be ordered with the context's other work on the device (one stream,
  *     or events).  The request loop queues on the context stream; frame streams own
@@ -671,15 +671,15 @@ gr_status gr_denoise_tonemap_device(gr_ctx *ctx, const float *film, uint32_t sam
 
 /* Transport kernel selection for single-scene renders.  PLAIN: one thread per
  * (pixel, sample) tuple, the reference kernel's launch shape.  WAVEFRONT and REGEN are
- * retired schedules (a global-queue wavefront engine, ~0.3x, and per-warp path
- * regeneration, 0.91x of STAGED on B200): both values are accepted and run AUTO's
- * choice.  STAGED: PLAIN's launch shape
- * with paths capped at 12 bounces; the ones still alive are parked and resumed, packed
- * densely, by a second kernel (capped at 20, then a third), so warps stop waiting on
- * a few long paths (+24-28% from 4 M tuples per launch up, e.g. the c2 frame).  AUTO
- * (default): STAGED for launches of at least GR_AUTO_STAGED_MIN_TUPLES tuples, PLAIN
- * below, where STAGED's extra launches and tails cost more than they save (measured
- * on B200: PLAIN 1.2x faster at 0.26 M tuples, STAGED 1.09x faster at 1.05 M).
+ * retired schedules: both values are accepted and run AUTO's choice.  STAGED: blocks of
+ * 512 threads (256 for clear isotropic stones) that hold one path per thread, run each
+ * bounce together and refill when half of their paths have ended, in three launches: the
+ * tuples, then the paths that outlive eight times the schedule's first cap while a block
+ * drains, then those past eight times the second (1.85-2.4x the time per sample of the
+ * earlier one-path-per-thread stages).  AUTO (default): STAGED for launches of at least
+ * GR_AUTO_STAGED_MIN_TUPLES tuples; below, PLAIN with 4 to 32 paths per warp, or the first
+ * of STAGED's launches alone (scenes with birefringence or absorption from 2^18 tuples,
+ * frosted / scattering / biaxial ones from 2^17).
  * Results are identical (same arithmetic per path). */
 #define GR_KERNEL_PLAIN 0u
 #define GR_KERNEL_WAVEFRONT 1u
@@ -696,21 +696,22 @@ gr_status gr_denoise_tonemap_device(gr_ctx *ctx, const float *film, uint32_t sam
 gr_status gr_set_kernel(gr_ctx *ctx, uint32_t kernel);
 
 /* The staged schedule of a resident scene's renders: bounce caps of stages 1 and 2 and
- * the resident blocks per SM the kernels' register allocation targets (9, 10, 12 or 16:
- * 56, 48, 40 or 32 registers per thread).  Every schedule gives the same films; the
- * fastest depends on the stone (measured on B200: caps 12 / 20 on the c2 brilliant,
- * 8 / 16 on the c3 emerald, 3.8% faster there; 16 blocks per SM 6-8% faster than 9 on
- * both).  From the scene's second staged gr_render_resident call on, calls are timed with
+ * the resident blocks per SM the kernels' register allocation targets, in blocks of 128
+ * threads (9, 10, 12 or 16; rounded down to whole blocks of 256 or 512).  Every schedule
+ * gives the same films; the fastest depends on the stone (measured on B200: 16 blocks on
+ * the clear brilliant, 12 on the dichroic emerald, 3-9% apart; the caps act only on paths
+ * longer than eight times their value).  From the scene's second staged
+ * gr_render_resident call on, calls are timed with
  * device events as trials, in two rounds: caps 12 / 20 at each blocks-per-SM target, then
  * caps 8 / 16 and 16 / 28 at the fastest target; the schedule with the least time per
  * tuple is kept for the scene and entered in the context's tuning table.  Writes zeros
  * while the choice is still open (the built-in schedule, caps 12 / 20 at 16 blocks per
- * SM, runs meanwhile).  Batched launches (gr_render_batch, the request loop) run each
- * scene with its chosen first cap (their continuation stage is uncapped); gr_accumulate
+ * SM for clear isotropic stones and 12 for others, runs meanwhile).  Batched launches (gr_render_batch, the request loop) run each
+ * scene with its chosen first cap, at 12 blocks per SM (their continuation stage is uncapped); gr_accumulate
  * and gr_accumulate_device choose the same way per stone (planes, finishes, material,
  * depth, flags and environment kind; not the view); a frame stream uses its scene's schedule as chosen when
  * the stream opened.  Scenes that need the frosted / scattering / biaxial kernels run
- * those at 9 blocks per SM whatever the schedule's target.  gr_scene_stage_caps reports
+ * those at 9 blocks per SM (two of 512 threads) whatever the schedule's target.  gr_scene_stage_caps reports
  * the caps alone. */
 gr_status gr_scene_stage_caps(gr_ctx *ctx, uint64_t scene_id, uint32_t *cap_first, uint32_t *cap_second);
 gr_status gr_scene_schedule(gr_ctx *ctx, uint64_t scene_id, uint32_t *cap_first, uint32_t *cap_second,

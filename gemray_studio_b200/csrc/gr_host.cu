@@ -195,7 +195,7 @@ gr_status validate_scene(const gr_scene *sc) {
 
 
 // Whether the transport of this scene stays finite: every number it reads is finite and
-// bounded, and the refractive indices over [380, 780] nm lie within (1.01, 8), so that no
+// bounded, and the refractive indices over [380, 780] nm lie within (1.0005, 8), so that no
 // Fresnel denominator vanishes.  The dispersion terms are monotonic in the wavelength
 // where they have no pole, so their values at the two ends bound them.  (A lat-long map is
 // checked texel by texel where it is read.)
@@ -251,14 +251,14 @@ static bool sane_scene(const gr_scene *sc, const SceneConst &S) {
         lo = sqrtf(fmaxf(lo, 0.0f));
         hi = sqrtf(fmaxf(hi, 0.0f));
     }
-    ok = ok && lo > 1.01f && hi < 8.0f;
+    ok = ok && lo > 1.0005f && hi < 8.0f;
     if (S.has_cauchy_e) {
         cauchy(S.cauchy_e, lo, hi);
     } else {
         lo += S.bire;
         hi += S.bire;
     }
-    return ok && lo > 1.01f && hi < 8.0f;
+    return ok && lo > 1.0005f && hi < 8.0f;
 }
 
 void encode_scene(const gr_scene *sc, SceneConst &S) {

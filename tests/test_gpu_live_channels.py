@@ -66,9 +66,9 @@ def test_live_channels_give_the_full_sums(renderer, name):
     assert np.nan_to_num(x, posinf=0.0).max() > 0.0
 
 
-@pytest.mark.parametrize("index", [1.0, 1.005, 0.7, 9.0])
-def test_indices_outside_the_range_match_the_oracle(renderer, oracle, index):
-    """These run the extension kernels; the bars are those of a clear isotropic stone."""
+@pytest.mark.parametrize("index", [1.0, 1.0002, 1.005, 0.7, 9.0])
+def test_indices_at_and_outside_the_range_match_the_oracle(renderer, oracle, index):
+    """All but 1.005 run the extension kernels; the bars are those of an isotropic stone."""
     from helpers import oracle_trace_samples
     sc = _scene("rb57", "Diamond", abi.GR_ENV_STUDIO, 16)
     sc.material = S.custom_material(index, 0.0, 0.0)

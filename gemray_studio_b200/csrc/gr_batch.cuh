@@ -78,14 +78,16 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     const LaunchRange R = G.R;
     const uint64_t first = (uint64_t)(blockIdx.x - G.block_begin) * chunk;
     float *xyz = G.xyz;
+    __shared__ HeroOrder H;
+    if (R.spp >= HERO_MIN_SPP) hero_order(H, R);
     Path P;
     run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K, true>(
         P, S, B, PL, PoolRange{first, min(first + chunk, R.n_tuples)}, G.stage_cap,
         ParkOut{park + G.park_off, G.park_cap, counts + s_seg},
         [&](Path &q, uint64_t t) {
-            uint32_t pixel, sample;
-            tuple_coords(R, t, pixel, sample);
-            path_init<K>(q, S, pixel, sample, (uint32_t)t);
+            uint32_t px, s;
+            hero_coords(R, H, t, px, s);
+            path_init<K>(q, S, R.first_pixel + px, R.sample_offset + s, px * R.spp + s);
         },
         [&](const Path &q) { store_sample(xyz, q, path_finish<1, false, K, EXTRAS>(q, S, B)); });
 }

@@ -116,7 +116,8 @@ __device__ __forceinline__ void store_sample(float *__restrict__ xyz, const Path
 // classes of 16 nm.  Chromatic termination leaves neighbouring heroes the same number of live
 // channels, and a warp runs its channel loops as often as its richest path: 288.8 -> 275.1 ms
 // on the 1080p brilliant at 256 spp, 144.6 -> 140.7 at 128, 4.23 -> 4.16 at 256^2 and 64 spp,
-// 36.9 -> 37.0 at 32 spp, so from 64 samples on.  Grouping the classes over several pixels
+// 36.9 -> 37.0 at 32 spp, so from 64 samples on; 64 batched stones of 32 to 512 spp 27.5 ->
+// 26.7.  Grouping the classes over several pixels
 // lost more than it gained (38.9 ms at 32 spp).
 constexpr uint32_t HERO_CLASSES = 25, HERO_MIN_SPP = 64;
 struct HeroOrder {

@@ -195,14 +195,22 @@ gr_status validate_scene(const gr_scene *sc) {
 
 
 // Whether the transport of this scene stays finite: every number it reads is finite and
-// bounded, and the refractive indices over [380, 780] nm lie within (1.0005, 8), so that no
-// Fresnel denominator vanishes.  The dispersion terms are monotonic in the wavelength
-// where they have no pole, so their values at the two ends bound them.  (A lat-long map is
-// checked texel by texel where it is read.)
+// bounded, no absorption is negative, and the refractive indices over [380, 780] nm lie
+// within (1.0005, 8), so that no Fresnel denominator vanishes.  The dispersion terms are
+// monotonic in the wavelength where they have no pole, so their values at the two ends bound
+// them.  (A lat-long map is checked texel by texel where it is read.)
 static bool sane_scene(const gr_scene *sc, const SceneConst &S) {
     bool ok = true;
     auto within = [&ok](float v, float most) { ok = ok && fabsf(v) <= most; };  // false for NaN
     auto within_n = [&](const float *v, size_t n, float most) { for (size_t i = 0; i < n; ++i) within(v[i], most); };
+    // A gain (a negative absorption or path scale) grows the Stokes vectors by up to e^88 a
+    // segment, past the finite range after two.  The rounding of a dichroic stone's absorption
+    // (2^-24 of it, of either sign) is no such gain while the whole is within 1e4.
+    float absorption = 0.0f;
+    auto lossy = [&](float v) {
+        ok = ok && v >= 0.0f;
+        absorption += v;
+    };
     within_n(S.cam_o, 3, 1e6f);
     within_n(S.cam_f, 3, 1e6f);
     within_n(S.cam_r, 3, 1e6f);
@@ -210,7 +218,6 @@ static bool sane_scene(const gr_scene *sc, const SceneConst &S) {
     within(S.fov_tan, 1e6f);
     if (sc->planes) within_n(&sc->planes[0].normal[0], (size_t)sc->n_planes * 4, 1e6f);
     within_n(S.c_axis, 3, 1e6f);
-    within(S.path_scale, 1e6f);
     within(S.edge_radius, 1e6f);
     within_n(S.uni_rgb, 3, 1e15f);
     within(S.temp_k, 1e15f);
@@ -219,14 +226,21 @@ static bool sane_scene(const gr_scene *sc, const SceneConst &S) {
     for (const auto *bands : {S.o_bands, S.e_bands}) {
         const uint32_t n = bands == S.o_bands ? S.n_o_bands : S.n_e_bands;
         for (uint32_t i = 0; i < n; ++i) {
-            within_n(bands[i], 3, 1e6f);
+            within_n(bands[i], 2, 1e6f);
+            lossy(bands[i][2]);
             ok = ok && fabsf(bands[i][1]) >= 1e-3f;
         }
     }
+    float most_o = 0.0f, most_e = 0.0f;
     for (uint32_t i = 0; i < S.ext_n; ++i) {
-        within(sc->material_ext->alpha_o_table[i], 1e6f);
-        within(sc->material_ext->alpha_e_table[i], 1e6f);
+        const float o = sc->material_ext->alpha_o_table[i], e = sc->material_ext->alpha_e_table[i];
+        ok = ok && o >= 0.0f && e >= 0.0f;  // false for NaN
+        most_o = fmaxf(most_o, o);
+        most_e = fmaxf(most_e, e);
     }
+    lossy(most_o);
+    lossy(most_e);
+    ok = ok && S.path_scale >= 0.0f && S.path_scale <= 1e6f && absorption * S.path_scale <= 1e4f;
     if (S.ext_n) ok = ok && S.ext_step >= 1e-6f && fabsf(S.ext_first) <= 1e6f;
     // bounds of n (Cauchy) or n^2 (Sellmeier) from each term's values at both ends
     const float ends[2] = {0.380f * 0.380f, 0.780f * 0.780f};

@@ -31,6 +31,7 @@ __global__ void __launch_bounds__(128) k_guide_pass(SceneConst S, const float4 *
                                                     int32_t *__restrict__ facet) {
     extern __shared__ float4 s_planes[];
     Planes PL = stage_plane_set(s_planes, gplanes, S.n_planes);
+    PL.small = S.small_planes != 0;
     const V3 o = ld3(S.cam_o);
     stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), o);
     const uint64_t n_px = (uint64_t)S.width * S.height, step = (uint64_t)gridDim.x * blockDim.x;
@@ -275,6 +276,7 @@ gr_status guide_device(gr_ctx *ctx, const gr_scene *sc, float *depth, float *nor
     S.width_f = (float)sc->width;
     S.height_f = (float)sc->height;
     S.n_planes = sc->n_planes;
+    S.small_planes = grh::planes_small(sc->planes, sc->n_planes);
     gr_status st = ctx->dn_planes.reserve((size_t)(sc->n_planes ? sc->n_planes : 1) * sizeof(float4));
     if (st != GR_OK) return st;
     if (sc->n_planes)

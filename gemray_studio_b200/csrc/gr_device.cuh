@@ -71,6 +71,7 @@ struct SceneConst {
     float d_beta_alpha;
     uint32_t has_beta, n_b_bands;
     float b_bands[GR_MAX_BANDS][3];
+    uint32_t small_planes;  // every component of every normal within 1e6 (planes_small)
     uint32_t sane;  // every input finite, no gain, every index in (1.0005, 8) (sane_scene)
 };
 

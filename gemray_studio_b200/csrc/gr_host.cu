@@ -194,6 +194,13 @@ gr_status validate_scene(const gr_scene *sc) {
 }
 
 
+uint32_t planes_small(const gr_plane *planes, uint32_t n) {
+    bool ok = true;
+    for (uint32_t i = 0; planes && i < n; ++i)
+        for (float v : planes[i].normal) ok = ok && fabsf(v) <= 1e6f;  // false for NaN
+    return ok ? 1u : 0u;
+}
+
 // Whether the transport of this scene stays finite: every number it reads is finite and
 // bounded, no absorption is negative, and the refractive indices over [380, 780] nm lie
 // within (1.0005, 8), so that no Fresnel denominator vanishes.  The dispersion terms are
@@ -359,6 +366,7 @@ void encode_scene(const gr_scene *sc, SceneConst &S) {
     S.map_w = sc->env.latlong_w;
     S.map_h = sc->env.latlong_h;
     S.flags = sc->flags;
+    S.small_planes = planes_small(sc->planes, sc->n_planes);
     S.sane = sane_scene(sc, S) ? 1u : 0u;
 }
 

@@ -28,6 +28,10 @@ gr_status metrics_device(const gr_plane *planes, uint32_t n_planes, const gr_mat
 // Device scratch bytes metrics_device needs (a scratch at least this large never grows).
 size_t metrics_scratch_bytes(uint32_t n_planes, uint32_t n_poses);
 
+// 1 if every component of every normal is within 1e6 (gr_host.cu): what the scans that order
+// planes by approximate keys need (Planes::small, gr_trace.cuh).
+uint32_t planes_small(const gr_plane *planes, uint32_t n);
+
 // The fixed scratch of gr_render_resident_static (gr_static.cu): its address on
 // `device` (the current device), looked up once per device.  Returns a cudaError_t.
 constexpr int kStaticMaxDevices = 64;

@@ -39,6 +39,12 @@ __device__ __forceinline__ Planes stage_plane_set(float4 *sp, const float4 *__re
     __syncthreads();
     return Planes{sp, pairs, n};
 }
+// The planes of a scene: X kernels take scenes of any planes, the default ones small planes.
+template <bool X> __device__ __forceinline__ Planes stage_scene_planes(float4 *sp, const SceneConst &S, const SceneBuffers &B) {
+    Planes PL = stage_plane_set(sp, B.planes, S.n_planes);
+    if (X) PL.small = S.small_planes != 0;
+    return PL;
+}
 
 // The camera's table of the staged planes (intersect_camera) at ct, camera_smem_bytes(n):
 // built by the first warp, one plane per lane; the whole block calls.
@@ -49,7 +55,7 @@ __device__ __forceinline__ void stage_camera_table(Planes &PL, float4 *ct, V3 o)
             const float4 p = PL.aos[i];
             return p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z);
         };
-        uint32_t n1 = 0, bad = 0;
+        uint32_t n1 = 0, bad = PL.small ? 0u : 1u;
         float min1 = 3.0e38f, min2 = 3.0e38f;
         for (uint32_t b = 0; b < PL.n; b += 32u) {
             const bool on = b + lane < PL.n;

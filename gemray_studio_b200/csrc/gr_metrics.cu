@@ -132,9 +132,10 @@ __host__ __device__ __forceinline__ bool cell_uv(int ix, int iz, float &u, float
 __global__ void __launch_bounds__(128) k_metric_traces(const PoseConst *__restrict__ poses, uint32_t n_poses,
                                                        const uint16_t *__restrict__ cells, uint32_t n_cells,
                                                        const float4 *__restrict__ gplanes, uint32_t n_planes,
-                                                       MetricTrace *__restrict__ out) {
+                                                       uint32_t small, MetricTrace *__restrict__ out) {
     extern __shared__ float4 s_planes[];
-    const Planes PL = stage_plane_set(s_planes, gplanes, n_planes);
+    Planes PL = stage_plane_set(s_planes, gplanes, n_planes);
+    PL.small = small != 0;
     const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= (uint64_t)n_poses * MTRACES * n_cells) return;
     const uint32_t ray = (uint32_t)(gid / n_cells), cell = cells[gid - (uint64_t)ray * n_cells];
@@ -396,7 +397,7 @@ gr_status metrics_device(const gr_plane *planes, uint32_t n_planes, const gr_mat
     const unsigned T = 128;
     grd::k_metric_traces<<<(unsigned)((threads + T - 1) / T), T, grd::planes_smem_bytes(n_planes), stream>>>(
         (const grd::PoseConst *)base, n_poses, (const uint16_t *)(base + L.cell_off), n_cells,
-        (const float4 *)(base + L.plane_off), n_planes, d_traces);
+        (const float4 *)(base + L.plane_off), n_planes, planes_small(planes, n_planes), d_traces);
     grd::k_metric_reduce<<<n_poses, grd::MREDUCE_THREADS, 0, stream>>>(d_traces, n_cells, d_out,
                                                                        (flags & GR_METRICS_FP64_SUMS) ? 1u : 0u);
     if (cudaGetLastError() != cudaSuccess) return GR_ECUDA;

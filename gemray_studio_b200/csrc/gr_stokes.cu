@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K_ANY>(), pool_blocks(MB,
     k_trace_stokes(SceneConst S, SceneBuffers B, LaunchRange R, float *__restrict__ xyz, float4 *__restrict__ iquv,
                    unsigned long long *work) {
     extern __shared__ float4 s_planes[];
-    Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
+    Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
     stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), ld3(S.cam_o));
     Path P;
     run_pool<pool_threads<EXTRAS, K_ANY>(), EXTRAS, K_ANY, true>(

@@ -308,6 +308,12 @@ struct Planes {
     const float4 *pairs;  // ceil(n / 2) x 2 float4, interleaved as above
     uint32_t n;
     const float4 *cam = nullptr;  // the camera's table (stage_camera_table), if staged
+    // Every normal's components are within 1e6, so that the scans that order planes by
+    // approximate keys (intersect_inside, intersect_camera) have finite ones: |denom| of a unit
+    // direction is below 2e6 and their factors are at most 1e30.  A larger denom may overflow,
+    // and an infinite key with an index in its low bits is a NaN, which the minima pass over.
+    // Such sets take the general scan.  (Scenes of the default kernels are all within it.)
+    bool small = true;
 };
 
 __host__ __device__ constexpr size_t planes_smem_bytes(uint32_t n) {
@@ -432,6 +438,7 @@ constexpr int SCAN_UNROLL = GR_SCAN_UNROLL;
 #endif
 constexpr int CAM_UNROLL = GR_CAM_UNROLL;
 __device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, float &t_hit, int &idx_hit) {
+    if (!PL.small) return SCAN_UNDECIDED;
     const f32x2 dx = pk2(d.x, d.x), dy = pk2(d.y, d.y), dz = pk2(d.z, d.z);
     const f32x2 ox = pk2(o.x, o.x), oy = pk2(o.y, o.y), oz = pk2(o.z, o.z);
     const uint32_t n2 = (PL.n + 1u) & ~1u;
@@ -467,7 +474,7 @@ __device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, fl
 // (side > 0, entered where the ray hits) and those it is not (side < 0, left), with rs =
 // -1 / side, and a ray needs only denom: u = denom * rs = 1 / t orders both lists.  The entry
 // facet has the least u of the first list, the exit the greatest of the second.  Sides of
-// zero or without a clear sign turn the table off.
+// zero or without a clear sign, and planes that are not small, turn the table off.
 // Table: a header (pairs of the first list, of both, bound of u below which a plane of the
 // first / second list may count as parallel), then per pair {nx0, nx1, ny0, ny1}, {nz0, nz1,
 // rs0, rs1}, {bias0, bias1, index0, index1}; the bias takes an odd list's padding out.

@@ -25,7 +25,7 @@ template <bool EXTRAS>
 __global__ void __launch_bounds__(TRACE_THREADS) k_trace_events(SceneConst S, SceneBuffers B, LaunchRange R,
                                                                 EventRec rec) {
     extern __shared__ float4 s_planes[];
-    const Planes PL = stage_plane_set(s_planes, B.planes, S.n_planes);
+    const Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= R.n_tuples) return;
     EventRec r = rec;
@@ -148,14 +148,15 @@ __global__ void k_case_bank(uint32_t bank, SceneConst S, SceneBuffers B, const f
 
 // The transport's clip (paired shared-memory scan) for one ray per thread.
 __global__ void k_intersect_rays(const float4 *__restrict__ planes, uint32_t n_planes, const float *__restrict__ rays,
-                                 uint32_t n, float *__restrict__ t_out, int32_t *__restrict__ facet_out) {
+                                 uint32_t n, uint32_t small, float *__restrict__ t_out, int32_t *__restrict__ facet_out) {
     extern __shared__ float4 s_planes[];
-    const Planes PL = stage_plane_set(s_planes, planes, n_planes);
+    Planes PL = stage_plane_set(s_planes, planes, n_planes);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float *r = rays + 6 * (size_t)i;
     float t = 0.0f;
     int idx = -1;
+    PL.small = small && fabsf(r[3]) <= 1.0f && fabsf(r[4]) <= 1.0f && fabsf(r[5]) <= 1.0f;  // any direction is taken
     const bool hit = intersect_from<false>(PL, true, v3(r[0], r[1], r[2]), v3(r[3], r[4], r[5]), t, idx);
     t_out[i] = hit ? t : 0.0f;
     facet_out[i] = hit ? idx : -1;
@@ -287,7 +288,8 @@ gr_status gr_intersect_rays(gr_ctx *ctx, const gr_plane *planes, uint32_t n_plan
     if (n_planes) GR_CUDA(cudaMemcpyAsync(base, planes, (size_t)n_planes * 16, cudaMemcpyHostToDevice, ctx->stream));
     GR_CUDA(cudaMemcpyAsync(base + o_rays, rays, (size_t)n * 24, cudaMemcpyHostToDevice, ctx->stream));
     grd::k_intersect_rays<<<(n + 127) / 128, 128, grd::planes_smem_bytes(n_planes), ctx->stream>>>(
-        (const float4 *)base, n_planes, (const float *)(base + o_rays), n, (float *)(base + o_t), (int32_t *)(base + o_f));
+        (const float4 *)base, n_planes, (const float *)(base + o_rays), n, grh::planes_small(planes, n_planes), (float *)(base + o_t),
+        (int32_t *)(base + o_f));
     GR_CUDA(cudaGetLastError());
     GR_CUDA(cudaMemcpyAsync(t, base + o_t, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     GR_CUDA(cudaMemcpyAsync(facet, base + o_f, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));

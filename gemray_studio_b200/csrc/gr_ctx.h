@@ -128,8 +128,10 @@ struct gr_ctx {
     int sm_count = 0;
     grh::DeviceBuffer xyz, film, planes, map, ext, counter, rgba, metrics;
     int kernel_mode = GR_KERNEL_AUTO;
-    // pooled kernels' park buffer (a header of counters, then parked path records)
-    grh::DeviceBuffer park;
+    // pooled kernels' park buffer (a header of counters, then parked path records); the header
+    // of AUTO's small pooled launches, allocated with the context, is a buffer of its own: they
+    // park nothing, allocate nothing in a call, and a captured one outlives the park buffer's growth
+    grh::DeviceBuffer park, pool_head;
     // Optional per-launch timing of the trace and fold kernels (CUDA events on the
     // launch stream); read back by gr_timing_read.
     bool timing = false;

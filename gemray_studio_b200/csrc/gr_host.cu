@@ -546,7 +546,7 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
     }
     if (mode == GR_KERNEL_STAGED) {
         const uint64_t slots = pool_alone ? 0 : staged_park_slots(R.n_tuples, ctx->sm_count);
-        grh::DeviceBuffer &pk = park_buf ? *park_buf : ctx->park;
+        grh::DeviceBuffer &pk = park_buf ? *park_buf : (pool_alone ? ctx->pool_head : ctx->park);
         gr_status st = pk.reserve(pool_alone ? kParkHeader : staged_park_bytes(R.n_tuples, ctx->sm_count));
         if (st != GR_OK) return st;
         GR_CUDA(cudaMemsetAsync(pk.ptr, 0, kParkHeader, stream));
@@ -828,6 +828,12 @@ gr_status gr_create(gr_ctx **out, const gr_create_opts *opts) {
         delete ctx;
         return fail(GR_ECUDA, "cudaStreamCreate failed: %s", cudaGetErrorString(e));
     }
+    const gr_status head = ctx->pool_head.reserve(grh::kParkHeader);
+    if (head != GR_OK) {
+        cudaStreamDestroy(ctx->stream);
+        delete ctx;
+        return head;
+    }
     ctx->sm_count = prop.multiProcessorCount;
     char buf[512];
     snprintf(buf, sizeof(buf), "%.256s (CUDA, sm_%d%d, %d SMs)", prop.name, prop.major, prop.minor, prop.multiProcessorCount);
@@ -861,6 +867,7 @@ gr_status gr_destroy(gr_ctx *ctx) {
         ctx->rgba.release();
         ctx->metrics.release();
         ctx->park.release();
+        ctx->pool_head.release();
         for (grh::DeviceBuffer *b : {&ctx->dn_a, &ctx->dn_b, &ctx->dn_n, &ctx->dn_g, &ctx->dn_in, &ctx->dn_out,
                                      &ctx->dn_planes})
             b->release();

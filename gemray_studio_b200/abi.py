@@ -253,6 +253,7 @@ EXPORTS = [
     ("gr_device_code_version", C.c_int, [_ctx_p, C.POINTER(C.c_uint32), C.POINTER(C.c_uint32)]),
     ("gr_intersect_rays", C.c_int, [_ctx_p, C.c_void_p, C.c_uint32, C.POINTER(C.c_float), C.c_uint32,
                                     C.POINTER(C.c_float), C.POINTER(C.c_int32)]),
+    ("gr_parked_counts", C.c_int, [_ctx_p, C.POINTER(C.c_uint32), C.POINTER(C.c_uint32), C.c_uint32]),
     ("gr_optical_metrics", C.c_int, [_ctx_p, C.c_void_p, C.c_uint32, C.POINTER(gr_material), C.POINTER(gr_pose),
                                      C.c_uint32, C.c_uint32, C.POINTER(gr_metrics_out)]),
     ("gr_angular_profile", C.c_int, [_ctx_p, C.c_void_p, C.c_uint32, C.POINTER(gr_material), C.c_float, C.c_float,

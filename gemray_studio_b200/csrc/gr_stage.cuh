@@ -154,7 +154,12 @@ __device__ __forceinline__ void run_pool(Path &P, const SceneConst &S, const Sce
             if (mask) {  // warp-uniform
                 const uint32_t lane = threadIdx.x & 31u, leader = __ffs((int)mask) - 1;
                 uint32_t slot = 0;
-                if (lane == leader) slot = atomicAdd(out.count, (unsigned)__popc(mask));
+                if (lane == leader) {
+                    // A full buffer is not asked again: such paths come here at every bounce, and
+                    // the 32-bit count has to stay below the slots plus the resident threads.
+                    slot = *(volatile unsigned int *)out.count;
+                    if (slot < out.cap) slot = atomicAdd(out.count, (unsigned)__popc(mask));
+                }
                 slot = __shfl_sync(0xffffffffu, slot, leader) + __popc(mask & ((1u << lane) - 1u));
                 if (want && slot < out.cap) {  // a full buffer: the path runs on here
                     copy_record<ROWS>(out.park[slot], P);

@@ -9,6 +9,7 @@
 // own functions, so what is checked is what renders.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -268,6 +269,19 @@ gr_status gr_device_code_version(gr_ctx *ctx, uint32_t *binary_version, uint32_t
     GR_CUDA(cudaFuncGetAttributes(&a, grd::k_case_bank));
     *binary_version = (uint32_t)a.binaryVersion;
     *ptx_version = (uint32_t)a.ptxVersion;
+    return GR_OK;
+}
+
+gr_status gr_parked_counts(gr_ctx *ctx, uint32_t *single, uint32_t *batch, uint32_t n_batch) {
+    if (!ctx || !single || (n_batch && !batch)) return fail(GR_EINVAL, "NULL argument");
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    GR_CUDA(cudaSetDevice(ctx->device));
+    single[0] = single[1] = 0;
+    std::memset(batch, 0, (size_t)n_batch * sizeof(uint32_t));
+    GR_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (ctx->park.ptr) GR_CUDA(cudaMemcpy(single, ctx->park.ptr, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    const size_t bytes = std::min(ctx->batch_park.cap, (size_t)n_batch * sizeof(uint32_t));
+    if (bytes) GR_CUDA(cudaMemcpy(batch, ctx->batch_park.ptr, bytes, cudaMemcpyDeviceToHost));
     return GR_OK;
 }
 

@@ -385,6 +385,13 @@ gr_status gr_device_code_version(gr_ctx *ctx, uint32_t *binary_version, uint32_t
 gr_status gr_intersect_rays(gr_ctx *ctx, const gr_plane *planes, uint32_t n_planes, const float *rays, uint32_t n,
                             float *t, int32_t *facet);
 
+/* The park slots that the context's last pooled launches asked for (paths that outlived eight
+ * times their cap in a draining block, whether or not there was room): stages 1 and 2 of the
+ * last staged single-scene trace in `single`, and the first n_batch segments of the last
+ * batched launch.  Waits for the context's stream; launches on other streams have to have
+ * ended. */
+gr_status gr_parked_counts(gr_ctx *ctx, uint32_t *single, uint32_t *batch, uint32_t n_batch);
+
 /* ---- optical metrics ------------------------------------------------------------ */
 
 /* = GemOpticalMetrics (color/metrics.rs:33-39). */

@@ -128,9 +128,7 @@ struct gr_ctx {
     int sm_count = 0;
     grh::DeviceBuffer xyz, film, planes, map, ext, counter, rgba, metrics;
     int kernel_mode = GR_KERNEL_AUTO;
-    // pooled kernels' park buffer (a header of counters, then parked path records); the header
-    // of AUTO's small pooled launches, allocated with the context, is a buffer of its own: they
-    // park nothing, allocate nothing in a call, and a captured one outlives the park buffer's growth
+    // pooled kernels' parked path records, and their counters (allocated with the context)
     grh::DeviceBuffer park, pool_head;
     // Optional per-launch timing of the trace and fold kernels (CUDA events on the
     // launch stream); read back by gr_timing_read.
@@ -274,10 +272,11 @@ StageCapTune &accum_tune(gr_ctx *ctx, const gr_scene *sc);
 // The gr_accumulate tuning key of a scene (its stone, not its view).
 uint64_t stone_key(const gr_scene *sc);
 int trace_kernel_launches(int mode, const SceneConst &S, uint64_t n_tuples);
-// Park slots of a pooled trace of n_tuples tuples on sm_count SMs: what its resident threads
-// can hold, since only a draining pool parks; and the bytes of the park buffer (a header of
-// counters and both stages' records).
-uint64_t staged_park_slots(uint64_t n_tuples, int sm_count);
+// Park slots of a stage of a pooled trace of n_tuples tuples on sm_count SMs: none where no
+// path can outlive the drain limit of its cap, else what its resident threads can hold, since
+// only a draining pool parks; and the most bytes a trace of that size takes (counters and both
+// stages' records).
+uint64_t staged_park_slots(uint64_t n_tuples, int sm_count, uint32_t max_bounces, uint32_t cap);
 size_t staged_park_bytes(uint64_t n_tuples, int sm_count);
 gr_status launch_fold(const float *xyz, uint32_t n_pixels, uint32_t spp, uint32_t first_pixel, float *film,
                       uint32_t kahan, cudaStream_t stream);

@@ -482,17 +482,34 @@ int trace_kernel_launches(int mode, const SceneConst &S, uint64_t n_tuples) {
     return staged ? 3 : 1;  // stages 1, 2 and 3
 }
 
-uint64_t staged_park_slots(uint64_t n_tuples, int sm_count) {
+uint64_t staged_park_slots(uint64_t n_tuples, int sm_count, uint32_t max_bounces, uint32_t cap) {
+    if (max_bounces / grd::DRAIN_CAPS < cap) return 0;
     const uint64_t resident = (uint64_t)(sm_count > 0 ? sm_count : 1) * 2048u;  // threads per SM
     return std::max<uint64_t>(1, std::min(n_tuples, resident));
 }
 
-// The park buffer's header: parked counts at 0, the sorted kernel's tuple counter at 8, the
+// The counters of a launch: parked counts at 0, the sorted kernel's tuple counter at 8, the
 // pooled stages' item counters at 64.
 constexpr size_t kParkHeader = 256, kParkWork = 64;
 
 size_t staged_park_bytes(uint64_t n_tuples, int sm_count) {
-    return 2 * (size_t)staged_park_slots(n_tuples, sm_count) * sizeof(grd::Path) + kParkHeader;
+    return 2 * (size_t)staged_park_slots(n_tuples, sm_count, GR_MAX_BOUNCES, 1) * sizeof(grd::Path) + kParkHeader;
+}
+
+// Where a launch's counters and parked records lie: in the caller's buffer one after the
+// other, or the counters with the context (allocated with it, so that a captured launch that
+// parks nothing keeps no pointer to a buffer that grows) and the records in its park buffer.
+static gr_status place_park(gr_ctx *ctx, DeviceBuffer *park_buf, uint64_t slots, char **head, grd::Path **records) {
+    const size_t bytes = (size_t)slots * sizeof(grd::Path);
+    DeviceBuffer &pk = park_buf ? *park_buf : ctx->park;
+    const size_t want = park_buf ? kParkHeader + bytes : bytes;
+    if (want) {
+        const gr_status st = pk.reserve(want);
+        if (st != GR_OK) return st;
+    }
+    *head = (char *)(park_buf ? pk.ptr : ctx->pool_head.ptr);
+    *records = (grd::Path *)((char *)pk.ptr + (park_buf ? kParkHeader : 0));
+    return GR_OK;
 }
 
 // Trace tuples [0, R.n_tuples) of one chunk into xyz (device).
@@ -537,25 +554,25 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
                      : launch_single_general(K, S, B, R, xyz, stream, nullptr);
     }
     if (mode == GR_KERNEL_SORTED) {
-        // the tuple counter of the sorted blocks sits in the park buffer's header, so a
-        // frame stream (own park buffer and stream) never shares it with the context
-        grh::DeviceBuffer &pk = park_buf ? *park_buf : ctx->park;
-        gr_status st = pk.reserve(256);
+        // a frame stream (own park buffer and stream) never shares the blocks' tuple counter
+        // with the context
+        char *head;
+        grd::Path *none;
+        const gr_status st = place_park(ctx, park_buf, 0, &head, &none);
         if (st != GR_OK) return st;
-        return launch_single_clear(K, S, B, R, xyz, stream, nullptr, (unsigned int *)pk.ptr + 2, ctx->sm_count);
+        return launch_single_clear(K, S, B, R, xyz, stream, nullptr, (unsigned int *)head + 2, ctx->sm_count);
     }
     if (mode == GR_KERNEL_STAGED) {
-        const uint64_t slots = pool_alone ? 0 : staged_park_slots(R.n_tuples, ctx->sm_count);
-        grh::DeviceBuffer &pk = park_buf ? *park_buf : (pool_alone ? ctx->pool_head : ctx->park);
-        gr_status st = pk.reserve(pool_alone ? kParkHeader : staged_park_bytes(R.n_tuples, ctx->sm_count));
-        if (st != GR_OK) return st;
-        GR_CUDA(cudaMemsetAsync(pk.ptr, 0, kParkHeader, stream));
         StagedLaunch sl;
-        sl.counts = (unsigned int *)pk.ptr;
-        sl.work = (unsigned long long *)((char *)pk.ptr + kParkWork);
-        sl.park1 = (grd::Path *)((char *)pk.ptr + kParkHeader);
-        sl.park2 = sl.park1 + slots;
-        sl.cap1 = sl.cap2 = slots;
+        sl.cap1 = pool_alone ? 0 : staged_park_slots(R.n_tuples, ctx->sm_count, S.max_bounces, caps.first);
+        sl.cap2 = sl.cap1 ? staged_park_slots(R.n_tuples, ctx->sm_count, S.max_bounces, caps.second) : 0;
+        char *head;
+        const gr_status st = place_park(ctx, park_buf, sl.cap1 + sl.cap2, &head, &sl.park1);
+        if (st != GR_OK) return st;
+        GR_CUDA(cudaMemsetAsync(head, 0, kParkHeader, stream));
+        sl.counts = (unsigned int *)head;
+        sl.work = (unsigned long long *)(head + kParkWork);
+        sl.park2 = sl.park1 + sl.cap1;
         sl.cap_first = caps.first;
         sl.cap_second = caps.second;
         sl.blocks = caps.blocks;

@@ -279,7 +279,7 @@ gr_status gr_parked_counts(gr_ctx *ctx, uint32_t *single, uint32_t *batch, uint3
     single[0] = single[1] = 0;
     std::memset(batch, 0, (size_t)n_batch * sizeof(uint32_t));
     GR_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (ctx->park.ptr) GR_CUDA(cudaMemcpy(single, ctx->park.ptr, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    GR_CUDA(cudaMemcpy(single, ctx->pool_head.ptr, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost));
     const size_t bytes = std::min(ctx->batch_park.cap, (size_t)n_batch * sizeof(uint32_t));
     if (bytes) GR_CUDA(cudaMemcpy(batch, ctx->batch_park.ptr, bytes, cudaMemcpyDeviceToHost));
     return GR_OK;

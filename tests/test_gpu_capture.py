@@ -1,7 +1,8 @@
-"""Renders captured into a CUDA graph: AUTO's launches below its staged size allocate nothing
+"""Device memory of renders, and renders captured into a CUDA graph: AUTO's launches below its staged size allocate nothing
 once the context's XYZ scratch has their size, whichever kernel they take (the plain one, or
 from 2^17 / 2^18 tuples the pool alone), and a captured one stays valid after a larger staged
-render has made the context grow its park buffer."""
+render has made the context grow its park buffer.  A staged launch takes park slots only
+where its depth lets a path outlive the drain limit."""
 from __future__ import annotations
 
 import ctypes as C
@@ -62,4 +63,37 @@ def test_small_launches_can_be_captured(engine_lib, material, w, h):
     del graph
     for i in (sid, big):
         r.lib.gr_scene_release(r.ctx, i)
+    r.close()
+
+
+def test_a_shallow_staged_launch_takes_no_park_slots(engine_lib):
+    """2^19 tuples at depth 32: the XYZ scratch (6 MiB) and counters.  A captured one stays
+    valid when a deep render makes the context allocate its park buffer."""
+    r = GpuFrameRenderer()
+    shallow, deep = _scene("Tourmaline", 1024, 512), _scene("Tourmaline", 1024, 512)
+    shallow.max_bounces, deep.max_bounces = 32, 512
+    n = 1024 * 512
+    a, b = _upload(r, shallow), _upload(r, deep)
+    for i in (a, b):  # no schedule trials
+        assert r.lib.gr_scene_set_schedule(r.ctx, i, 12, 20, 12) == abi.GR_OK
+    film = torch.zeros((n, 3), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    assert r.lib.gr_render_resident(r.ctx, a, 0, 1, film.data_ptr(), None) == abi.GR_OK
+    r.synchronize()
+    want = film.cpu().numpy()
+    assert free - torch.cuda.mem_get_info()[0] < 32 << 20
+    graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=s):
+        st = r.lib.gr_render_resident(r.ctx, a, 0, 1, film.data_ptr(), C.c_void_p(s.cuda_stream))
+    assert st == abi.GR_OK, r.lib.gr_last_error_string()
+    assert r.lib.gr_render_resident(r.ctx, b, 0, 1, film.data_ptr(), None) == abi.GR_OK
+    r.synchronize()
+    film.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(film.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    del graph
+    r.lib.gr_scene_release(r.ctx, a)
+    r.lib.gr_scene_release(r.ctx, b)
     r.close()

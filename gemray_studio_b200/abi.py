@@ -130,7 +130,7 @@ class gr_batch_item(C.Structure):
 
 
 GR_BATCH_GRAPH = 0x1
-GR_SCHEDULE_SET = 2
+GR_SCHEDULE_SET = 3
 # staged schedules a stone chooses between: cap pairs x blocks per SM
 SCHEDULE_CAP_PAIRS = ((12, 20), (8, 16), (16, 28))
 SCHEDULE_BLOCKS = (9, 10, 12, 16)

@@ -738,7 +738,7 @@ gr_status gr_scene_set_schedule(gr_ctx *ctx, uint64_t scene_id, uint32_t cap_fir
  * GR_ENOTFOUND if it cannot be read) and gives open scenes their entries.  With the
  * environment variable GR_TUNING_CACHE set to a path, gr_create loads that file and
  * gr_destroy saves to it: a per-device schedule cache across processes. */
-#define GR_SCHEDULE_SET 2
+#define GR_SCHEDULE_SET 3 /* 3: measured on the pooled kernels; 1 and 2 on those before them */
 gr_status gr_tuning_save(gr_ctx *ctx, const char *path);
 gr_status gr_tuning_load(gr_ctx *ctx, const char *path, uint32_t *n_loaded);
 gr_status gr_tuning_count(gr_ctx *ctx, uint32_t *n_entries);

@@ -399,12 +399,13 @@ __device__ __forceinline__ bool scan_plane(float denom, float side, int i, float
 // negative for exactly those planes, and the exit facet has the least v.  v carries the
 // plane's index in its low 9 bits, so one minimum finds both, and the second least v
 // says whether the order is certain: rcp.approx (1 ulp), the product and the 9 bits
-// move v by less than 2^-13.9 of itself, so when the second is not within 2^-11 of the
-// least, the winner's exact quotient is the strictly least one whatever the rounding.
-// Only that quotient is then divided, from the same sums as the reference.
+// (511 ulp) move v by less than 6.12e-5 of itself, so when the second is not within
+// SCAN_MARGIN of the least, the winner's exact quotient is the strictly least one whatever
+// the rounding.  Only that quotient is then divided, from the same sums as the reference.
+// Facets within the margin (an edge) are settled by their exact quotients .
 // Everything else -- a side that is not clearly negative (the origin on or outside a
-// plane, a NaN), no plane to leave through, two facets within 2^-11 (an edge) -- returns
-// SCAN_UNDECIDED, and the general scan decides.
+// plane, a NaN), no plane to leave through -- returns SCAN_UNDECIDED, and the general scan
+// decides.
 //
 // Why: the general scan's updates and divisions are branches, and among the lanes of a
 // warp some lane takes them at nearly every plane, so the warp pays for them 73 times a
@@ -437,6 +438,13 @@ constexpr int SCAN_UNROLL = GR_SCAN_UNROLL;
 #define GR_CAM_UNROLL 1
 #endif
 constexpr int CAM_UNROLL = GR_CAM_UNROLL;
+__device__ __forceinline__ float plane_denom(const float4 &p, V3 d) { return (p.x * d.x + p.y * d.y) + p.z * d.z; }
+__device__ __forceinline__ float plane_side(const float4 &p, V3 o) { return p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z); }
+
+// Two keys further apart than this have quotients in their order: (1 + e) / (1 - e) for e =
+// 6.12e-5, and 2^-22 for the quotients' own rounding.
+constexpr float SCAN_MARGIN = 1.3e-4f;
+
 __device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, float &t_hit, int &idx_hit) {
     if (!PL.small) return SCAN_UNDECIDED;
     const f32x2 dx = pk2(d.x, d.x), dy = pk2(d.y, d.y), dz = pk2(d.z, d.z);
@@ -458,14 +466,25 @@ __device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, fl
         second = min3(second, hi, fmaxf(best, lo));
         best = fminf(best, lo);
     }
-    if (!(side_max < -1e-30f) || !(best < -1e-20f) || !(second > best * (1.0f - 4.8828125e-4f))) return SCAN_UNDECIDED;
+    if (!(side_max < -1e-30f) || !(best < -1e-20f)) return SCAN_UNDECIDED;
     const int idx = (int)(__float_as_uint(best) & SCAN_INDEX_MASK);
-    const float4 p = PL.aos[idx];
-    const float denom = (p.x * d.x + p.y * d.y) + p.z * d.z;
-    const float side = p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z);
+    const float denom = plane_denom(PL.aos[idx], d);
     if (!(denom > 1e-7f)) return SCAN_UNDECIDED;
-    t_hit = (-side) / denom;
+    t_hit = (-plane_side(PL.aos[idx], o)) / denom;
     idx_hit = idx;
+    const float bound = best * (1.0f - SCAN_MARGIN);
+    if (!(second > bound)) {  // the quotients of every plane that may be the least, in plane order
+        float least = 1e30f;
+#pragma unroll 1
+        for (uint32_t i = 0; i < PL.n; ++i) {
+            const float4 p = PL.aos[i];
+            const float den = plane_denom(p, d), side = plane_side(p, o);
+            if (!(scan_key(den * rcp_approx(side), i) <= bound) || !(den > 1e-7f)) continue;
+            const float t = (-side) / den;
+            if (t < least) { least = t; idx_hit = (int)i; }
+        }
+        t_hit = least;
+    }
     return t_hit > 1e-4f ? SCAN_HIT : SCAN_MISS;
 }
 
@@ -480,8 +499,8 @@ __device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, fl
 // rs0, rs1}, {bias0, bias1, index0, index1}; the bias takes an odd list's padding out.
 __host__ __device__ constexpr size_t camera_smem_bytes(uint32_t n) { return (size_t)(1u + 3u * (n / 2u + 1u)) * 16u; }
 
-// As intersect_inside: keys with the index in 9 bits, exact quotient for the winner alone, and
-// SCAN_UNDECIDED within 2^-11 of a tie or of a parallel plane.
+// As intersect_inside: keys with the index in 9 bits, exact quotients for the winner and what
+// ties with it alone, and SCAN_UNDECIDED near the outline or a parallel plane.
 // Every primary ray took the general scan; with the table the brilliant at 32 spp went from
 // 39.0 to 37.7 ms (16 blocks), the emerald from 38.8 to 38.0 (12), 64 batched stones from 28.3
 // to 27.3, guide pass + filter + tone map of 1920x1080 from 1.143 to 1.120 ms.
@@ -519,15 +538,31 @@ __device__ __forceinline__ int intersect_camera(const Planes &PL, V3 d, V3 o, fl
     }
     if (near < -head.z) return SCAN_MISS;  // a plane the origin is beyond, and the ray leaves
     if (!(near > head.z) || !(far > head.w)) return SCAN_UNDECIDED;
-    if (near < far * (1.0f - 4.8828125e-4f)) return SCAN_MISS;  // leaves before it has entered
-    if (!(near > far * (1.0f + 4.8828125e-4f)) || !(near2 > near * (1.0f + 4.8828125e-4f))) return SCAN_UNDECIDED;
+    if (near < far * (1.0f - SCAN_MARGIN)) return SCAN_MISS;  // leaves before it has entered
+    if (!(near > far * (1.0f + SCAN_MARGIN))) return SCAN_UNDECIDED;
     const int idx = (int)(__float_as_uint(near) & SCAN_INDEX_MASK);
-    const float4 p = PL.aos[idx];
-    const float denom = (p.x * d.x + p.y * d.y) + p.z * d.z;
-    const float side = p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z);
-    t_hit = (-side) / denom;
+    const float denom = plane_denom(PL.aos[idx], d);
+    t_hit = (-plane_side(PL.aos[idx], o)) / denom;
     idx_hit = idx;
-    return denom < -1e-7f && t_hit > 1e-4f && t_hit < 1e29f ? SCAN_HIT : SCAN_UNDECIDED;
+    if (!(denom < -1e-7f) || !(t_hit > 1e-4f) || !(t_hit < 1e29f)) return SCAN_UNDECIDED;
+    const float bound = near * (1.0f + SCAN_MARGIN);
+    if (!(near2 > bound)) {  // the quotients of every plane that may be entered last, in plane order
+        float most = -1e30f;
+#pragma unroll 1
+        for (q = PL.cam + 1; q < q1; q += 3) {
+            float k[2];
+            keys(q, k[0], k[1]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (!(k[h] <= bound)) continue;
+                const int i = (int)(__float_as_uint(k[h]) & SCAN_INDEX_MASK);
+                const float t = (-plane_side(PL.aos[i], o)) / plane_denom(PL.aos[i], d);
+                if (t > most) { most = t; idx_hit = i; }
+            }
+        }
+        t_hit = most;
+    }
+    return SCAN_HIT;
 }
 
 // The reference clip (intersect.rs:93-132) in FP64, t rounded back to f32: the

@@ -4,8 +4,8 @@
 // The reference's film is XYZ only (renderer/gpu/frame.rs:799-814); its transport
 // carries a Stokes vector per hero-wavelength channel (optics/polarization.rs:4-66
 // StokesVector, spectral_transport.wgsl transport_main's per-channel state) and drops
-// it at the end of the path.  The Stokes variant of the plain kernel keeps it: per
-// tuple the luminance-weighted Stokes vector of the escaping light (path_finish<.., true>,
+// it at the end of the path.  The Stokes variants of the plain and the pooled kernel keep it:
+// per tuple the luminance-weighted Stokes vector of the escaping light (path_finish<.., true>,
 // gr_trace.cuh), folded per pixel in sample order like the XYZ film.
 #include <cuda_runtime.h>
 
@@ -15,7 +15,7 @@
 #include <vector>
 
 #include "gr_ctx.h"
-#include "gr_stage.cuh"
+#include "gr_transport.cuh"
 
 using grh::fail;
 
@@ -43,6 +43,26 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K_ANY>(), pool_blocks(MB,
             store_sample(xyz, q, path_finish<1, true, K_ANY, EXTRAS>(q, S, B, &s4));
             iquv[p_tuple(q)] = s4;
         });
+}
+
+// The plain kernel (gr_transport.cuh) writing XYZ and IQUV, for launches that leave the chip
+// idle.
+template <bool EXTRAS>
+__global__ void __launch_bounds__(TRACE_THREADS, GR_TRACE_MIN_BLOCKS)
+    k_trace_stokes_plain(SceneConst S, SceneBuffers B, LaunchRange R, float *__restrict__ xyz, float4 *__restrict__ iquv,
+                         uint32_t lanes) {
+    extern __shared__ float4 s_planes[];
+    const Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
+    const uint64_t t = plain_tuple(lanes, R.n_tuples);
+    if (t >= R.n_tuples) return;
+    uint32_t pixel, sample;
+    tuple_coords(R, t, pixel, sample);
+    Path P;
+    path_init(P, S, pixel, sample, (uint32_t)t);
+    NoCounters nc;
+    float4 s4;
+    store_sample(xyz, P, trace_path<NoCounters, false, EXTRAS, K_ANY, true>(P, S, B, PL, nc, &s4));
+    iquv[t] = s4;
 }
 
 // One warp per pixel: the pixel's spp Stokes vectors summed in sample order from zero,
@@ -78,6 +98,13 @@ __global__ void k_stokes_fold(const float4 *__restrict__ iquv, uint32_t n_pixels
 #define GR_STOKES_BLOCKS 12
 #endif
 constexpr int kStokesBlocks = GR_STOKES_BLOCKS;
+// Launches below these sizes run the plain kernel: the pool's 512-thread blocks leave most of
+// the chip idle there and wait at their barriers for the longest scan of the block.  Measured
+// (us of a call, plain / pool): birefringent emerald 16,384 tuples 380 / 553, 131,072 624 /
+// 750, 262,144 878 / 885, 393,216 1523 / 1396; clear brilliant 65,536 472 / 740, 262,144 835 /
+// 1058, 524,288 1670 / 1693; quartz cube 2,048 155 / 258, 131,072 370 / 366; frosted biaxial
+// 16,384 964 / 1337, 65,536 1386 / 1368, 131,072 1970 / 1562.
+constexpr uint64_t kStokesPlain = 1u << 18, kStokesPlainExtras = 1u << 16;
 
 extern "C" {
 
@@ -114,7 +141,7 @@ gr_status gr_accumulate_stokes(gr_ctx *ctx, const gr_scene *sc, uint32_t sample_
     if (st != GR_OK) return st;
     float *txyz = (float *)ctx->xyz.ptr;
     float4 *tiquv = (float4 *)((char *)ctx->xyz.ptr + toff);
-    const size_t smem = grd::planes_smem_bytes(S.n_planes) + grd::camera_smem_bytes(S.n_planes);
+    const size_t plane_smem = grd::planes_smem_bytes(S.n_planes), smem = plane_smem + grd::camera_smem_bytes(S.n_planes);
     st = ctx->counter.reserve(64);
     if (st != GR_OK) return st;
     for (uint64_t first = 0; first < n_pixels; first += chunk_pixels) {
@@ -125,15 +152,25 @@ gr_status gr_accumulate_stokes(gr_ctx *ctx, const gr_scene *sc, uint32_t sample_
         R.sample_offset = sample_offset;
         R.spp = spp;
         R.n_tuples = np * spp;
+        const bool extras = grd::needs_extras(S);
         constexpr int T = grd::pool_threads<true, grd::K_ANY>();
         const uint64_t resident = (uint64_t)(ctx->sm_count > 0 ? ctx->sm_count : 1) * grd::pool_blocks(kStokesBlocks, T);
         const unsigned blocks = (unsigned)std::min<uint64_t>(resident, (R.n_tuples + T - 1) / T);
-        GR_CUDA(cudaMemsetAsync(ctx->counter.ptr, 0, sizeof(unsigned long long), ctx->stream));
-        unsigned long long *work = (unsigned long long *)ctx->counter.ptr;
-        if (grd::needs_extras(S))
-            grd::k_trace_stokes<true, kStokesBlocks><<<blocks, T, smem, ctx->stream>>>(S, B, R, txyz, tiquv, work);
-        else
-            grd::k_trace_stokes<false, kStokesBlocks><<<blocks, T, smem, ctx->stream>>>(S, B, R, txyz, tiquv, work);
+        if (R.n_tuples < (extras ? kStokesPlainExtras : kStokesPlain)) {
+            const uint32_t lanes = grd::plain_lanes(R.n_tuples, false);
+            const unsigned grid = grd::plain_blocks(R.n_tuples, lanes);
+            if (extras)
+                grd::k_trace_stokes_plain<true><<<grid, grd::TRACE_THREADS, plane_smem, ctx->stream>>>(S, B, R, txyz, tiquv, lanes);
+            else
+                grd::k_trace_stokes_plain<false><<<grid, grd::TRACE_THREADS, plane_smem, ctx->stream>>>(S, B, R, txyz, tiquv, lanes);
+        } else {
+            GR_CUDA(cudaMemsetAsync(ctx->counter.ptr, 0, sizeof(unsigned long long), ctx->stream));
+            unsigned long long *work = (unsigned long long *)ctx->counter.ptr;
+            if (extras)
+                grd::k_trace_stokes<true, kStokesBlocks><<<blocks, T, smem, ctx->stream>>>(S, B, R, txyz, tiquv, work);
+            else
+                grd::k_trace_stokes<false, kStokesBlocks><<<blocks, T, smem, ctx->stream>>>(S, B, R, txyz, tiquv, work);
+        }
         GR_CUDA(cudaGetLastError());
         ctx->trace_launches += 1;
         st = grh::launch_fold(txyz, (uint32_t)np, spp, (uint32_t)first, film_x, (S.flags & GR_FLAG_KAHAN_FILM) ? 1u : 0u,

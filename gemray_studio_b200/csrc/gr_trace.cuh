@@ -1351,17 +1351,17 @@ __device__ __forceinline__ V3 path_finish(const Path &P, const SceneConst &S, co
     return von_kries(acc, S.wb);
 }
 
-// One whole path in the calling thread (the plain kernel's body).
-template <class CT, bool R = false, bool X = false, int K = K_ANY>
+// One whole path in the calling thread (the plain kernels' body).
+template <class CT, bool R = false, bool X = false, int K = K_ANY, bool STOKES = false>
 __device__ __forceinline__ V3 trace_path(Path &P, const SceneConst &S, const SceneBuffers &B, const Planes &PL,
-                                         CT &ct) {
+                                         CT &ct, float4 *iquv = nullptr) {
     while (state_bits(P) & F_ALIVE) {
         Event E;
         uint32_t ev = step_hit<1, CT, R, X, K>(P, S, B, PL, E, ct);
         if (ev == EV_REFLECT) step_reflect<1, CT, X, K>(P, S, E, ct);
         else if (ev == EV_REFRACT) step_refract<1, CT, X, K>(P, S, E, ct);
     }
-    return path_finish<1, false, K, X>(P, S, B);
+    return path_finish<1, STOKES, K, X>(P, S, B, iquv);
 }
 
 }  // namespace grd

@@ -9,6 +9,12 @@
 
 namespace grd {
 
+// The thread's tuple in a plain launch of `lanes` tuples per warp; `none` for the other lanes.
+__device__ __forceinline__ uint64_t plain_tuple(uint32_t lanes, uint64_t none) {
+    const uint32_t lane = threadIdx.x & 31u;
+    return lane < lanes ? ((uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u) * lanes + lane : none;
+}
+
 // Plain kernel: one thread traces one tuple start to finish, `lanes` tuples per warp -- the reference
 // kernel's launch shape (one invocation per (pixel, sample), spectral_transport.wgsl:
 // 672-691).  The Counters variant tallies events for the FLOP model; RESOLVE is the
@@ -22,9 +28,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_plain(SceneConst S,
                                                                uint32_t lanes = 32) {
     extern __shared__ float4 s_planes[];
     const Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
-    uint64_t t = R.n_tuples;
-    if ((threadIdx.x & 31u) < lanes)
-        t = ((uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u) * lanes + (threadIdx.x & 31u);
+    const uint64_t t = plain_tuple(lanes, R.n_tuples);
     CT ct;
     if constexpr (sizeof(CT) == sizeof(Counters)) {
         for (int i = 0; i < C_COUNT; ++i) ((Counters &)ct).c[i] = 0;

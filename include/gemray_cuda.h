@@ -259,7 +259,8 @@ gr_status gr_trace_samples(gr_ctx *ctx, const gr_scene *scene, uint32_t first_pi
  * 8 hero channels, with the XYZ sum's spectral-MIS weight w, normaliser and intensity
  * clamp, so I equals that sum's Y before white balance.  Q, U, V are in the frame of
  * the last plane of incidence; every per-sample vector has sqrt(Q^2+U^2+V^2) <= I up to
- * rounding.  Plain kernel; not with GR_FLAG_FP64_RESOLVE. */
+ * rounding.  The plain kernel below 2^18 tuples (2^16 for frosted, scattering or biaxial
+ * scenes), the pooled one from there; not with GR_FLAG_FP64_RESOLVE. */
 gr_status gr_accumulate_stokes(gr_ctx *ctx, const gr_scene *scene, uint32_t sample_offset, uint32_t spp,
                                float *accum_xyz, float *accum_stokes);
 

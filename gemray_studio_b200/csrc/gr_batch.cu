@@ -200,7 +200,7 @@ gr_status make_plan(gr_ctx *ctx, const grh::BatchItem *items, uint32_t n_items, 
             cur.seg_count++;
             cur.warps += np;
             cur.max_planes = std::max(cur.max_planes, rs->S.n_planes);
-            cur.extras = cur.extras || grd::needs_extras(rs->S);
+            cur.extras = cur.extras || grd::has_extensions(rs->S);
             used += g.R.n_tuples;
             next += np;
         }
@@ -230,13 +230,10 @@ gr_status launch_plan(const Plan &P, const grd::SceneSlot *slots, const grd::Bat
         if (L.extras) {
             grd::launch_batch_grids<true, grd::K_ANY, GR_TRACE_MIN_BLOCKS>(slots, segs + L.seg_first, L.seg_count, L.chunk, park,
                                                                            counts, L.blocks, L.park_blocks, smem, grd::camera_smem_bytes(L.max_planes), s);
-        } else if (L.K >= 0) {
+        } else {
             const gr_status st = grh::launch_batch_class(L.K, slots, segs + L.seg_first, L.seg_count, L.chunk, park, counts,
                                                          L.blocks, L.park_blocks, smem, grd::camera_smem_bytes(L.max_planes), s);
             if (st != GR_OK) return st;
-        } else {
-            grd::launch_batch_grids<false, grd::K_ANY, GR_TRACE_MIN_BLOCKS>(slots, segs + L.seg_first, L.seg_count, L.chunk, park,
-                                                                            counts, L.blocks, L.park_blocks, smem, grd::camera_smem_bytes(L.max_planes), s);
         }
         const unsigned T = 256;
         grd::k_fold_batch<<<(unsigned)((L.warps * 32 + T - 1) / T), T, 0, s>>>(segs + L.seg_first, L.seg_count);

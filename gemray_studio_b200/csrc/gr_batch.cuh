@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     __syncthreads();
     const SceneConst &S = s_slot.S;
     const SceneBuffers &B = s_slot.B;
-    Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
+    Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
     stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), ld3(S.cam_o));
     const LaunchRange R = G.R;
     const uint64_t first = (uint64_t)(blockIdx.x - G.block_begin) * chunk;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     __syncthreads();
     const SceneConst &S = s_slot.S;
     const SceneBuffers &B = s_slot.B;
-    const Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
+    const Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
     const Path *from = park + G.park_off;
     float *xyz = G.xyz;
     Path P;

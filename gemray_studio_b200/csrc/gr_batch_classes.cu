@@ -30,6 +30,8 @@ gr_status launch_batch_class(int K, const grd::SceneSlot *slots, const grd::Batc
         GR_BATCH_CASE(grd::k_env(GR_ENV_UNIFORM))
         GR_BATCH_CASE(grd::k_env(GR_ENV_STUDIO))
         GR_BATCH_CASE(grd::k_env(GR_ENV_LATLONG))
+        GR_BATCH_CASE(IC | grd::K_FULL)
+        GR_BATCH_CASE(grd::K_FULL)
     default: return fail(GR_EINVAL, "scene class %d has no batched kernels", K);
     }
 #undef GR_BATCH_CASE

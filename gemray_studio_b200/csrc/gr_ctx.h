@@ -222,7 +222,8 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
                        float *xyz, cudaStream_t stream, int mode, grh::DeviceBuffer *park = nullptr,
                        StageCaps caps = StageCaps{});
 // The compile-time scene class of a single-scene launch (gr_trace.cuh K_*): clear
-// isotropic stones (K_ISO | K_CLEAR) and the rest, each with its environment kind;
+// isotropic stones (K_ISO | K_CLEAR) and the rest, each with its environment kind, or with
+// K_FULL for scenes whose arithmetic may leave the finite range;
 // -1 for scenes the extension variant handles (frosted, scattering, biaxial).
 int scene_class(const SceneConst &S);
 // Park buffers, counters and schedule of a pooled single-scene trace (prepared by
@@ -238,13 +239,15 @@ struct StagedLaunch {
     bool alone;       // the first launch only, nothing parked (small launches under AUTO)
 };
 // The plain kernel (st == NULL) or the three staged launches of scene class K
-// (gr_single_clear.cu / gr_single_general.cu).
+// (gr_single_clear.cu / gr_single_general.cu / gr_single_full.cu, whose blocks per SM are fixed).
 // sorted_work != NULL: the block-sorted kernel (gr_sorted.cuh) instead, its tuple counter.
 gr_status launch_single_clear(int K, const SceneConst &S, const grd::SceneBuffers &B, const grd::LaunchRange &R,
                               float *xyz, cudaStream_t stream, const StagedLaunch *st,
                               unsigned int *sorted_work = nullptr, int sm_count = 0);
 gr_status launch_single_general(int K, const SceneConst &S, const grd::SceneBuffers &B, const grd::LaunchRange &R,
                                 float *xyz, cudaStream_t stream, const StagedLaunch *st);
+gr_status launch_single_full(int K, const SceneConst &S, const grd::SceneBuffers &B, const grd::LaunchRange &R,
+                             float *xyz, cudaStream_t stream, const StagedLaunch *st);
 // The kernel a launch of n_tuples tuples runs in `mode` (AUTO resolved by size), and
 // how many kernel launches that trace makes.
 int resolve_kernel(int mode, uint64_t n_tuples);

@@ -76,13 +76,16 @@ struct SceneConst {
 };
 
 // Scenes that need the extension instantiation of the transport kernels: frosted facets,
-// volume scattering, biaxial materials -- and scenes whose arithmetic may leave the finite
-// range, since the extension instantiation alone computes every term and every channel
-// (live_only, gr_trace.cuh).  Every other scene runs the default instantiation, which
-// contains none of that code.
-__host__ __device__ inline bool needs_extras(const SceneConst &S) {
-    return S.any_frosted || S.sigma_s > 0.0f || S.biaxial || !S.sane;
+// volume scattering, biaxial materials.  Every other scene runs the default instantiation,
+// which contains none of that code.
+__host__ __device__ inline bool has_extensions(const SceneConst &S) {
+    return S.any_frosted || S.sigma_s > 0.0f || S.biaxial;
 }
+// Scenes whose arithmetic may leave the finite range are among those that the default
+// instantiation's live-channel form does not cover: the extension instantiation and the scene
+// class K_FULL (gr_trace.cuh) compute every term and every channel.  The verification kernels
+// take the extension instantiation for both.
+__host__ __device__ inline bool needs_extras(const SceneConst &S) { return has_extensions(S) || !S.sane; }
 
 struct SceneBuffers {
     const float4 *planes;      // n_planes

@@ -460,9 +460,9 @@ int resolve_kernel(int mode, uint64_t n_tuples) {
 }
 
 int scene_class(const SceneConst &S) {
-    if (grd::needs_extras(S)) return -1;
-    const bool iso = !S.anisotropic && !S.biaxial, clear = !S.absorbing;
-    return ((iso && clear) ? (grd::K_ISO | grd::K_CLEAR) : 0) | grd::k_env(S.env_mode);
+    if (grd::has_extensions(S)) return -1;
+    const int K = (!S.anisotropic && !S.absorbing) ? (grd::K_ISO | grd::K_CLEAR) : 0;
+    return S.sane ? K | grd::k_env(S.env_mode) : K | grd::K_FULL;
 }
 
 // The kernel a single-scene launch of this scene runs: GR_KERNEL_SORTED only for clear
@@ -470,7 +470,7 @@ int scene_class(const SceneConst &S) {
 static int scene_kernel(int mode, const SceneConst &S, uint64_t n_tuples) {
     if (mode == GR_KERNEL_SORTED) {
         const int K = scene_class(S);
-        const bool ok = K >= 0 && (K & grd::K_CLEAR) && S.max_bounces > 0 && !(S.flags & GR_FLAG_FP64_RESOLVE);
+        const bool ok = K >= 0 && (K & grd::K_CLEAR) && !(K & grd::K_FULL) && S.max_bounces > 0 && !(S.flags & GR_FLAG_FP64_RESOLVE);
         if (!ok) mode = GR_KERNEL_AUTO;
     }
     return resolve_kernel(mode, n_tuples);
@@ -512,8 +512,14 @@ static gr_status place_park(gr_ctx *ctx, DeviceBuffer *park_buf, uint64_t slots,
     return GR_OK;
 }
 
-// Trace tuples [0, R.n_tuples) of one chunk into xyz (device).
+static gr_status launch_single(int K, const SceneConst &S, const grd::SceneBuffers &B, const grd::LaunchRange &R, float *xyz,
+                               cudaStream_t stream, const StagedLaunch *st) {
+    if (K & grd::K_FULL) return launch_single_full(K, S, B, R, xyz, stream, st);
+    return (K & grd::K_CLEAR) ? launch_single_clear(K, S, B, R, xyz, stream, st)
+                              : launch_single_general(K, S, B, R, xyz, stream, st);
+}
 
+// Trace tuples [0, R.n_tuples) of one chunk into xyz (device).
 gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers &B, const grd::LaunchRange &R,
                        float *xyz, cudaStream_t stream, int mode, grh::DeviceBuffer *park_buf, StageCaps caps) {
     if (caps.first == 0) caps = StageCaps{GR_STAGE_CAP, GR_STAGE_CAP2};
@@ -521,12 +527,15 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
     const int asked = mode;
     mode = scene_kernel(mode, S, R.n_tuples);
     size_t smem = grd::planes_smem_bytes(S.n_planes);
-    const bool extras = grd::needs_extras(S);
+    const bool extras = grd::has_extensions(S);
     const uint64_t plain_blocks = (R.n_tuples + grd::TRACE_THREADS - 1) / grd::TRACE_THREADS;
     if (S.flags & GR_FLAG_FP64_RESOLVE) {  // the re-solve variant exists for the plain kernel only
         if (extras)
             grd::k_trace_plain<grd::NoCounters, true, true><<<(unsigned)plain_blocks, grd::TRACE_THREADS, smem, stream>>>(
                 S, B, R, xyz, nullptr);
+        else if (!S.sane)
+            grd::k_trace_plain<grd::NoCounters, true, false, grd::K_FULL>
+                <<<(unsigned)plain_blocks, grd::TRACE_THREADS, smem, stream>>>(S, B, R, xyz, nullptr);
         else
             grd::k_trace_plain<grd::NoCounters, true><<<(unsigned)plain_blocks, grd::TRACE_THREADS, smem, stream>>>(
                 S, B, R, xyz, nullptr);
@@ -550,8 +559,7 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
             GR_CUDA(cudaGetLastError());
             return GR_OK;
         }
-        return clear ? launch_single_clear(K, S, B, R, xyz, stream, nullptr)
-                     : launch_single_general(K, S, B, R, xyz, stream, nullptr);
+        return launch_single(K, S, B, R, xyz, stream, nullptr);
     }
     if (mode == GR_KERNEL_SORTED) {
         // a frame stream (own park buffer and stream) never shares the blocks' tuple counter
@@ -578,9 +586,7 @@ gr_status launch_trace(gr_ctx *ctx, const SceneConst &S, const grd::SceneBuffers
         sl.blocks = caps.blocks;
         sl.sm_count = ctx->sm_count > 0 ? ctx->sm_count : 1;
         sl.alone = pool_alone;
-        if (!extras)
-            return clear ? launch_single_clear(K, S, B, R, xyz, stream, &sl)
-                         : launch_single_general(K, S, B, R, xyz, stream, &sl);
+        if (!extras) return launch_single(K, S, B, R, xyz, stream, &sl);
         grd::launch_pool<true, grd::K_ANY, GR_TRACE_MIN_BLOCKS>(S, B, R, xyz, stream, pool_launch(sl));
         GR_CUDA(cudaGetLastError());
         return GR_OK;

@@ -39,10 +39,12 @@ __device__ __forceinline__ Planes stage_plane_set(float4 *sp, const float4 *__re
     __syncthreads();
     return Planes{sp, pairs, n};
 }
-// The planes of a scene: X kernels take scenes of any planes, the default ones small planes.
-template <bool X> __device__ __forceinline__ Planes stage_scene_planes(float4 *sp, const SceneConst &S, const SceneBuffers &B) {
+// The planes of a scene: the extension kernels and those of class K_FULL take scenes of any
+// planes, the others small planes.
+template <bool X, int K = K_ANY>
+__device__ __forceinline__ Planes stage_scene_planes(float4 *sp, const SceneConst &S, const SceneBuffers &B) {
     Planes PL = stage_plane_set(sp, B.planes, S.n_planes);
-    if (X) PL.small = S.small_planes != 0;
+    if (X || (K & K_FULL)) PL.small = S.small_planes != 0;
     return PL;
 }
 

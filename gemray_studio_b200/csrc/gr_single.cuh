@@ -23,20 +23,24 @@ gr_status launch_staged_mb(const SceneConst &S, const grd::SceneBuffers &B, cons
     return GR_OK;
 }
 
-// The plain kernel (st == NULL, at the built-in GR_TRACE_MIN_BLOCKS), or the staged
-// launches at the blocks per SM the schedule asks for (kScheduleBlocks; 0 =
-// builtin_schedule_blocks).
+// The plain kernel at the built-in GR_TRACE_MIN_BLOCKS.
+template <int K>
+gr_status launch_plain_k(const SceneConst &S, const grd::SceneBuffers &B, const grd::LaunchRange &R, float *xyz,
+                         cudaStream_t stream) {
+    const size_t smem = grd::planes_smem_bytes(S.n_planes);
+    const uint32_t lanes = grd::plain_lanes(R.n_tuples, (K & grd::K_CLEAR) != 0);
+    grd::k_trace_plain<grd::NoCounters, false, false, K, GR_TRACE_MIN_BLOCKS>
+        <<<grd::plain_blocks(R.n_tuples, lanes), grd::TRACE_THREADS, smem, stream>>>(S, B, R, xyz, nullptr, lanes);
+    GR_CUDA(cudaGetLastError());
+    return GR_OK;
+}
+
+// The plain kernel (st == NULL), or the staged launches at the blocks per SM the schedule asks
+// for (kScheduleBlocks; 0 = builtin_schedule_blocks).
 template <int K>
 gr_status launch_single_k(const SceneConst &S, const grd::SceneBuffers &B, const grd::LaunchRange &R, float *xyz,
                           cudaStream_t stream, const StagedLaunch *st) {
-    if (!st) {
-        const size_t smem = grd::planes_smem_bytes(S.n_planes);
-        const uint32_t lanes = grd::plain_lanes(R.n_tuples, (K & grd::K_CLEAR) != 0);
-        grd::k_trace_plain<grd::NoCounters, false, false, K, GR_TRACE_MIN_BLOCKS>
-            <<<grd::plain_blocks(R.n_tuples, lanes), grd::TRACE_THREADS, smem, stream>>>(S, B, R, xyz, nullptr, lanes);
-        GR_CUDA(cudaGetLastError());
-        return GR_OK;
-    }
+    if (!st) return launch_plain_k<K>(S, B, R, xyz, stream);
     static_assert(kScheduleBlockCount == 4, "one launch per kScheduleBlocks entry");
     switch (st->blocks ? st->blocks : builtin_schedule_blocks(K)) {
         case kScheduleBlocks[0]: return launch_staged_mb<K, kScheduleBlocks[0]>(S, B, R, xyz, stream, st);

@@ -23,15 +23,15 @@ namespace grd {
 
 // The pooled kernel (gr_stage.cuh) writing XYZ (the same arithmetic as the film's kernels) and
 // IQUV per tuple; nothing is parked.
-template <bool EXTRAS, int MB>
-__global__ void __launch_bounds__(pool_threads<EXTRAS, K_ANY>(), pool_blocks(MB, pool_threads<EXTRAS, K_ANY>()))
+template <bool EXTRAS, int K, int MB>
+__global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, pool_threads<EXTRAS, K>()))
     k_trace_stokes(SceneConst S, SceneBuffers B, LaunchRange R, float *__restrict__ xyz, float4 *__restrict__ iquv,
                    unsigned long long *work) {
     extern __shared__ float4 s_planes[];
-    Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
+    Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
     stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), ld3(S.cam_o));
     Path P;
-    run_pool<pool_threads<EXTRAS, K_ANY>(), EXTRAS, K_ANY, true>(
+    run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K, true>(
         P, S, B, PL, PoolQueue{work, R.n_tuples}, 0xFFFFFFFFu, ParkOut{nullptr, 0, nullptr},
         [&](Path &q, uint64_t t) {
             uint32_t pixel, sample;
@@ -40,19 +40,19 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K_ANY>(), pool_blocks(MB,
         },
         [&](const Path &q) {
             float4 s4;
-            store_sample(xyz, q, path_finish<1, true, K_ANY, EXTRAS>(q, S, B, &s4));
+            store_sample(xyz, q, path_finish<1, true, K, EXTRAS>(q, S, B, &s4));
             iquv[p_tuple(q)] = s4;
         });
 }
 
 // The plain kernel (gr_transport.cuh) writing XYZ and IQUV, for launches that leave the chip
 // idle.
-template <bool EXTRAS>
+template <bool EXTRAS, int K>
 __global__ void __launch_bounds__(TRACE_THREADS, GR_TRACE_MIN_BLOCKS)
     k_trace_stokes_plain(SceneConst S, SceneBuffers B, LaunchRange R, float *__restrict__ xyz, float4 *__restrict__ iquv,
                          uint32_t lanes) {
     extern __shared__ float4 s_planes[];
-    const Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
+    const Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
     const uint64_t t = plain_tuple(lanes, R.n_tuples);
     if (t >= R.n_tuples) return;
     uint32_t pixel, sample;
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, GR_TRACE_MIN_BLOCKS)
     path_init(P, S, pixel, sample, (uint32_t)t);
     NoCounters nc;
     float4 s4;
-    store_sample(xyz, P, trace_path<NoCounters, false, EXTRAS, K_ANY, true>(P, S, B, PL, nc, &s4));
+    store_sample(xyz, P, trace_path<NoCounters, false, EXTRAS, K, true>(P, S, B, PL, nc, &s4));
     iquv[t] = s4;
 }
 
@@ -90,8 +90,6 @@ __global__ void k_stokes_fold(const float4 *__restrict__ iquv, uint32_t n_pixels
     }
 }
 
-}  // namespace grd
-
 // Resident blocks per SM of the Stokes kernels, in blocks of 128 threads (384 x 256 emerald at
 // 64 spp: one path per thread 15.8 ms; pooled at 12 / 9 blocks 7.69 / 7.83).
 #ifndef GR_STOKES_BLOCKS
@@ -105,6 +103,25 @@ constexpr int kStokesBlocks = GR_STOKES_BLOCKS;
 // 1058, 524,288 1670 / 1693; quartz cube 2,048 155 / 258, 131,072 370 / 366; frosted biaxial
 // 16,384 964 / 1337, 65,536 1386 / 1368, 131,072 1970 / 1562.
 constexpr uint64_t kStokesPlain = 1u << 18, kStokesPlainExtras = 1u << 16;
+
+// One launch's samples.  work: the pooled kernel's tuple counter.
+template <bool EXTRAS, int K>
+void launch_stokes(const SceneConst &S, const SceneBuffers &B, const LaunchRange &R, float *xyz, float4 *iquv,
+                   unsigned long long *work, uint32_t sm_count, cudaStream_t s) {
+    const size_t smem = planes_smem_bytes(S.n_planes);
+    if (R.n_tuples < (EXTRAS ? kStokesPlainExtras : kStokesPlain)) {
+        const uint32_t lanes = plain_lanes(R.n_tuples, false);
+        k_trace_stokes_plain<EXTRAS, K><<<plain_blocks(R.n_tuples, lanes), TRACE_THREADS, smem, s>>>(S, B, R, xyz, iquv, lanes);
+        return;
+    }
+    cudaMemsetAsync(work, 0, sizeof(*work), s);
+    constexpr int T = pool_threads<EXTRAS, K>();
+    const uint64_t resident = (uint64_t)sm_count * pool_blocks(kStokesBlocks, T), need = (R.n_tuples + T - 1) / T;
+    k_trace_stokes<EXTRAS, K, kStokesBlocks><<<(unsigned)std::min(resident, need), T, smem + camera_smem_bytes(S.n_planes), s>>>(
+        S, B, R, xyz, iquv, work);
+}
+
+}  // namespace grd
 
 extern "C" {
 
@@ -141,7 +158,6 @@ gr_status gr_accumulate_stokes(gr_ctx *ctx, const gr_scene *sc, uint32_t sample_
     if (st != GR_OK) return st;
     float *txyz = (float *)ctx->xyz.ptr;
     float4 *tiquv = (float4 *)((char *)ctx->xyz.ptr + toff);
-    const size_t plane_smem = grd::planes_smem_bytes(S.n_planes), smem = plane_smem + grd::camera_smem_bytes(S.n_planes);
     st = ctx->counter.reserve(64);
     if (st != GR_OK) return st;
     for (uint64_t first = 0; first < n_pixels; first += chunk_pixels) {
@@ -152,25 +168,11 @@ gr_status gr_accumulate_stokes(gr_ctx *ctx, const gr_scene *sc, uint32_t sample_
         R.sample_offset = sample_offset;
         R.spp = spp;
         R.n_tuples = np * spp;
-        const bool extras = grd::needs_extras(S);
-        constexpr int T = grd::pool_threads<true, grd::K_ANY>();
-        const uint64_t resident = (uint64_t)(ctx->sm_count > 0 ? ctx->sm_count : 1) * grd::pool_blocks(kStokesBlocks, T);
-        const unsigned blocks = (unsigned)std::min<uint64_t>(resident, (R.n_tuples + T - 1) / T);
-        if (R.n_tuples < (extras ? kStokesPlainExtras : kStokesPlain)) {
-            const uint32_t lanes = grd::plain_lanes(R.n_tuples, false);
-            const unsigned grid = grd::plain_blocks(R.n_tuples, lanes);
-            if (extras)
-                grd::k_trace_stokes_plain<true><<<grid, grd::TRACE_THREADS, plane_smem, ctx->stream>>>(S, B, R, txyz, tiquv, lanes);
-            else
-                grd::k_trace_stokes_plain<false><<<grid, grd::TRACE_THREADS, plane_smem, ctx->stream>>>(S, B, R, txyz, tiquv, lanes);
-        } else {
-            GR_CUDA(cudaMemsetAsync(ctx->counter.ptr, 0, sizeof(unsigned long long), ctx->stream));
-            unsigned long long *work = (unsigned long long *)ctx->counter.ptr;
-            if (extras)
-                grd::k_trace_stokes<true, kStokesBlocks><<<blocks, T, smem, ctx->stream>>>(S, B, R, txyz, tiquv, work);
-            else
-                grd::k_trace_stokes<false, kStokesBlocks><<<blocks, T, smem, ctx->stream>>>(S, B, R, txyz, tiquv, work);
-        }
+        const uint32_t sm_count = ctx->sm_count > 0 ? ctx->sm_count : 1;
+        unsigned long long *work = (unsigned long long *)ctx->counter.ptr;
+        if (grd::has_extensions(S)) grd::launch_stokes<true, grd::K_ANY>(S, B, R, txyz, tiquv, work, sm_count, ctx->stream);
+        else if (!S.sane) grd::launch_stokes<false, grd::K_FULL>(S, B, R, txyz, tiquv, work, sm_count, ctx->stream);
+        else grd::launch_stokes<false, grd::K_ANY>(S, B, R, txyz, tiquv, work, sm_count, ctx->stream);
         GR_CUDA(cudaGetLastError());
         ctx->trace_launches += 1;
         st = grh::launch_fold(txyz, (uint32_t)np, spp, (uint32_t)first, film_x, (S.flags & GR_FLAG_KAHAN_FILM) ? 1u : 0u,

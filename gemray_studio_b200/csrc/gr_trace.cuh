@@ -79,6 +79,9 @@ constexpr int K_ANY = 0;
 constexpr int K_ISO = 1;        // S.anisotropic == 0 (and not biaxial)
 constexpr int K_CLEAR = 2;      // S.absorbing == 0: no absorption data at all
 constexpr int K_ENV_SHIFT = 2;  // bits 2-3: 0 = the environment kind at run time, else GR_ENV_* + 1
+// Every term and every channel, for scenes whose arithmetic may leave the finite range
+// (SceneConst::sane; the environment kind at run time).
+constexpr int K_FULL = 16;
 __host__ __device__ constexpr int k_env(uint32_t env) { return (int)(env + 1) << K_ENV_SHIFT; }
 template <int K> __device__ __forceinline__ bool aniso_k(const SceneConst &S) {
     return (K & K_ISO) ? false : (S.anisotropic != 0);
@@ -87,7 +90,8 @@ template <int K> __device__ __forceinline__ bool absorbing_k(uint32_t bits) {
     return (K & K_CLEAR) ? false : ((bits & F_ABSORBING) != 0);
 }
 template <int K> __device__ __forceinline__ uint32_t env_k(const SceneConst &S) {
-    return (K >> K_ENV_SHIFT) ? (uint32_t)((K >> K_ENV_SHIFT) - 1) : S.env_mode;
+    constexpr int env = (K >> K_ENV_SHIFT) & 3;
+    return env ? (uint32_t)(env - 1) : S.env_mode;
 }
 
 // EV_HANDLED: the bounce was completed inside step_hit (a frosted facet or a volume
@@ -167,15 +171,15 @@ template <> __device__ __forceinline__ void note_end<EventRec>(EventRec &r, uint
 // paths keep two or three of the eight: neighbours in wavelength bend within the
 // termination angle of the hero only near normal incidence, and the lanes of a warp
 // (samples of one pixel) enter through the same facet, so their counts agree.
-// The extension instantiation (X) and the event counters take all channels every time;
-// scenes whose factors might not be finite run the X kernels (SceneConst::sane).
+// The extension instantiation (X), the class K_FULL of scenes whose factors might not be
+// finite (SceneConst::sane) and the event counters take all channels every time.
 // What bounds these loops is issue and instruction fetch; skipping the dead channels
 // measured 479.9 ms against 554.5 on the 1080p brilliant (256 spp), 170.1 against 191.3 on
 // the 1024^2 dichroic emerald (96 spp), 5.65 against 6.53 on the 256^2 brilliant (64 spp).
-template <class CT, bool X> constexpr bool live_only = !X;
-template <bool X> constexpr bool live_only<Counters, X> = false;
-template <class CT, bool X> __device__ __forceinline__ uint32_t live_channels(uint32_t bits) {
-    return live_only<CT, X> ? (bits >> LIVE_SHIFT) & 0xFFu : 0xFFu;
+template <class CT, bool X, int K> constexpr bool live_only = !X && !(K & K_FULL);
+template <bool X, int K> constexpr bool live_only<Counters, X, K> = false;
+template <class CT, bool X, int K> __device__ __forceinline__ uint32_t live_channels(uint32_t bits) {
+    return live_only<CT, X, K> ? (bits >> LIVE_SHIFT) & 0xFFu : 0xFFu;
 }
 template <bool LIVE, int U, class F> __device__ __forceinline__ void each_channel(uint32_t live, F f) {
     if constexpr (LIVE) {
@@ -919,7 +923,7 @@ __device__ __forceinline__ uint32_t step_facet(Path &P, const SceneConst &S, con
     uint32_t bits = state_bits(P);
     const uint32_t bounce = bits_bounce(bits);
     const bool inside = (bits & F_INSIDE) != 0;
-    const uint32_t live = live_channels<CT, X>(bits);
+    const uint32_t live = live_channels<CT, X, K>(bits);
     const V3 o = xyz(P.o_hero), d = xyz(P.d_seed), kk = xyz(P.k_state);
     if (bounce == 0) {  // the bounce index grows with every event: the first hit, once per path
         bits |= channel_tables<U, X, K>(P, S, B);
@@ -941,10 +945,10 @@ __device__ __forceinline__ uint32_t step_facet(Path &P, const SceneConst &S, con
     if (dot(cur_plane, cur_plane) > 1e-6f && dot(prev, prev) > 1e-6f) {
         float psi = signed_psi(prev, cur_plane, kk);
         float2 sc = m_sincos(2.0f * psi);
-        each_channel<live_only<CT, X>, ALL_UNROLL>(live, [&](int k) {
+        each_channel<live_only<CT, X, K>, ALL_UNROLL>(live, [&](int k) {
             float4 s = P.st[k];
             const Stokes in{s.x, s.y, s.z, s.w};
-            const Stokes r = live_only<CT, X> ? rotate_finite<(K & K_CLEAR) != 0>(in, sc.y, sc.x)
+            const Stokes r = live_only<CT, X, K> ? rotate_finite<(K & K_CLEAR) != 0>(in, sc.y, sc.x)
                                               : apply_rotation(in, sc.y, sc.x);
             P.st[k] = make_float4(r.i, r.q, r.u, r.v);
         });
@@ -963,7 +967,7 @@ __device__ __forceinline__ uint32_t step_facet(Path &P, const SceneConst &S, con
             // Every channel's alpha reads that channel's Stokes vector before it is
             // scaled, so computing and applying per channel is the reference's
             // two-pass loop (absorption.rs:123-140) in one pass.
-            each_channel<live_only<CT, X>, U>(live, [&](int k) {
+            each_channel<live_only<CT, X, K>, U>(live, [&](int k) {
                 float4 s4 = P.st[k];
                 Stokes s{s4.x, s4.y, s4.z, s4.w};
                 V3 e_hat = electric_field_direction(s, cur_plane, kk);
@@ -988,7 +992,7 @@ __device__ __forceinline__ uint32_t step_facet(Path &P, const SceneConst &S, con
         const float theta = theta_c<U>(kk, normal, cos_i, one_m_c2, n_o_hero, n_e_hero, ld3(S.c_axis), !inside);
         float2 sc = m_sincos(theta);
         const bool use_o = inside && !(bits & F_IS_E);
-        each_channel<live_only<CT, X>, U>(live, [&](int k) {
+        each_channel<live_only<CT, X, K>, U>(live, [&](int k) {
             float n_o = arr(P.n_o4, k);
             arr(E.n_med4, k) = use_o ? n_o : eff_e_index(n_o, n_o + arr(P.ne_d4, k), sc.x, sc.y);
         });
@@ -1064,9 +1068,9 @@ __device__ __forceinline__ void step_post(Path &P, const SceneConst &S, V3 hp, V
         bits = rng_draw(seed, bounce, MODE_COUPLING_STREAM) < 0.5f ? (bits | F_IS_E) : (bits & ~F_IS_E);
     if (bounce > 4) {
         tally(ct, C_ROULETTE);
-        const uint32_t live = live_channels<CT, X>(bits);
+        const uint32_t live = live_channels<CT, X, K>(bits);
         float mx = 0.0f;
-        each_channel<live_only<CT, X>, ALL_UNROLL>(live, [&](int k) { mx = fmaxf(mx, fmaxf(P.st[k].x, 0.0f)); });
+        each_channel<live_only<CT, X, K>, ALL_UNROLL>(live, [&](int k) { mx = fmaxf(mx, fmaxf(P.st[k].x, 0.0f)); });
         float q = clampf(mx, 0.05f, 1.0f);
         if (rng_draw(seed, bounce, RUSSIAN_ROULETTE_STREAM) > q) {
             tally(ct, C_ROULETTE_KILLS);
@@ -1075,7 +1079,7 @@ __device__ __forceinline__ void step_post(Path &P, const SceneConst &S, V3 hp, V
             return;
         }
         const float iq = 1.0f / q;
-        each_channel<live_only<CT, X>, ALL_UNROLL>(live, [&](int k) {
+        each_channel<live_only<CT, X, K>, ALL_UNROLL>(live, [&](int k) {
             float4 s = P.st[k];
             P.st[k] = make_float4(s.x * iq, s.y * iq, s.z * iq, s.w * iq);
         });
@@ -1163,8 +1167,8 @@ __device__ __forceinline__ void step_reflect(Path &P, const SceneConst &S, const
     // A TIR event applies each channel's matrix unscaled: the reflect branch's
     // `.scale(1 / r_unpol)` with factor 1.0 (x * 1.0f == x exactly).
     const float inv = hero_tir ? 1.0f : 1.0f / E.n_ru.w;
-    constexpr bool FIN = live_only<CT, X>, CLEAR = (K & K_CLEAR) != 0;
-    each_channel<live_only<CT, X>, U>(live_channels<CT, X>(bits), [&](int k) {
+    constexpr bool FIN = live_only<CT, X, K>, CLEAR = (K & K_CLEAR) != 0;
+    each_channel<live_only<CT, X, K>, U>(live_channels<CT, X, K>(bits), [&](int k) {
         const float nm = n_med<K>(P, E, k);
         const float n1k = inside ? nm : 1.0f, n2k = inside ? 1.0f : nm;
         const float etak = inside ? nm : 1.0f / nm;  // n1k / n2k: one of them is 1
@@ -1234,8 +1238,8 @@ __device__ __forceinline__ void step_refract(Path &P, const SceneConst &S, const
     const float tinv = 1.0f / (1.0f - ru);
     const float TOL = 1.0f - 1e-6f;
     uint32_t ended = 0u;  // channels terminated here
-    constexpr bool FIN = live_only<CT, X>, CLEAR = (K & K_CLEAR) != 0;
-    each_channel<live_only<CT, X>, U>(live_channels<CT, X>(bits), [&](int k) {
+    constexpr bool FIN = live_only<CT, X, K>, CLEAR = (K & K_CLEAR) != 0;
+    each_channel<live_only<CT, X, K>, U>(live_channels<CT, X, K>(bits), [&](int k) {
         const float n_o_k = arr(P.n_o4, k);
         const float n1k = inside ? n_med<K>(P, E, k) : 1.0f;
         const float n2k = ordinary_entry ? n_o_k : (inside ? 1.0f : n_med<K>(P, E, k));
@@ -1270,7 +1274,7 @@ __device__ __forceinline__ void step_refract(Path &P, const SceneConst &S, const
         }
         P.st[k] = make_float4(s.i, s.q, s.u, s.v);
     });
-    if (live_only<CT, X>) set_state_bits(P, bits & ~(ended << LIVE_SHIFT));
+    if (live_only<CT, X, K>) set_state_bits(P, bits & ~(ended << LIVE_SHIFT));
     step_post<CT, K, X>(P, S, hp, refr, final_dir, !inside, entering_aniso, use_e, ct);
 }
 
@@ -1312,8 +1316,9 @@ __device__ __forceinline__ V3 path_finish(const Path &P, const SceneConst &S, co
     // A dead channel, a path that did not escape and a black environment add zero: those
     // channels' colour matching and spectra are not formed (a map texel that is not
     // finite takes them all, as zero times it is no zero).
-    uint32_t live = live_channels<NoCounters, X>(state_bits(P));
-    if (!X) {
+    uint32_t live = live_channels<NoCounters, X, K>(state_bits(P));
+    constexpr bool LIVE = live_only<NoCounters, X, K>;
+    if (LIVE) {
         if (!escaped) {
             live = 0u;
         } else if (env_mode != GR_ENV_STUDIO) {
@@ -1323,7 +1328,7 @@ __device__ __forceinline__ V3 path_finish(const Path &P, const SceneConst &S, co
     }
     V3 acc = v3(0.f, 0.f, 0.f);
     float4 sk = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    each_channel<!X, U>(live, [&](int k) {
+    each_channel<LIVE, U>(live, [&](int k) {
         const float lam = lambda_k(hero, k);
         float rad = 0.0f, q = 0.0f, u = 0.0f, v = 0.0f;
         if (escaped) {

@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_plain(SceneConst S,
                                                                unsigned long long *__restrict__ tallies,
                                                                uint32_t lanes = 32) {
     extern __shared__ float4 s_planes[];
-    const Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
+    const Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
     const uint64_t t = plain_tuple(lanes, R.n_tuples);
     CT ct;
     if constexpr (sizeof(CT) == sizeof(Counters)) {
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     k_trace_pool(SceneConst S, SceneBuffers B, LaunchRange R, float *__restrict__ xyz, unsigned long long *work,
                  ParkOut out, uint32_t bounce_cap) {
     extern __shared__ float4 s_planes[];
-    Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
+    Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
     stage_camera_table(PL, s_planes + planes_smem_bytes(S.n_planes) / sizeof(float4), ld3(S.cam_o));
     __shared__ HeroOrder H;
     if (R.spp >= HERO_MIN_SPP) hero_order(H, R);
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
     const uint32_t n = min((uint32_t)*count_in, cap_in);
     if ((uint64_t)blockIdx.x * blockDim.x >= n) return;  // more blocks than parked paths fill
     extern __shared__ float4 s_planes[];
-    const Planes PL = stage_scene_planes<EXTRAS>(s_planes, S, B);
+    const Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
     Path P;
     run_pool<pool_threads<EXTRAS, K>(), EXTRAS, K, false>(
         P, S, B, PL, PoolQueue{work, n}, bounce_cap, out,

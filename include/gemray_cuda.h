@@ -719,7 +719,8 @@ gr_status gr_set_kernel(gr_ctx *ctx, uint32_t kernel);
  * and gr_accumulate_device choose the same way per stone (planes, finishes, material,
  * depth, flags and environment kind; not the view); a frame stream uses its scene's schedule as chosen when
  * the stream opened.  Scenes that need the frosted / scattering / biaxial kernels run
- * those at 9 blocks per SM (two of 512 threads) whatever the schedule's target.  gr_scene_stage_caps reports
+ * those at 9 blocks per SM (two of 512 threads) whatever the schedule's target, scenes with
+ * an index outside (1.0005, 8), a gain medium or huge inputs theirs at 12 (clear) or 9.  gr_scene_stage_caps reports
  * the caps alone. */
 gr_status gr_scene_stage_caps(gr_ctx *ctx, uint64_t scene_id, uint32_t *cap_first, uint32_t *cap_second);
 gr_status gr_scene_schedule(gr_ctx *ctx, uint64_t scene_id, uint32_t *cap_first, uint32_t *cap_second,

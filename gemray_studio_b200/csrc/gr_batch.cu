@@ -14,6 +14,7 @@
 // Launches are pooled like the single-scene renders (gr_stage.cuh): a k_trace_batch block runs
 // its pool over up to kBatchFills blocks' worth of one segment's tuples; k_trace_batch_cont
 // finishes the few paths that outlive its drain, one block's worth of one segment per block.
+// Small shallow launches run k_trace_batch_plain instead, one path per thread.
 //
 // With GR_BATCH_GRAPH the launch sequence is captured once as a CUDA graph and
 // replayed whenever the same batch shape recurs (same scenes, films, spp, frame sizes
@@ -59,6 +60,7 @@ struct Launch {
     uint32_t max_planes;
     bool extras;  // a segment's scene has frosted facets, scattering or a biaxial material
     uint32_t chunk;  // tuples one trace block runs
+    uint32_t lanes;  // tuples per warp in the plain form, 0: the pooled form
     uint64_t park_paths, park_blocks;  // park slots over the launch's segments, continuation blocks
     int K;        // the scene class of every segment (scene_class), -1: the extension kernels
 };
@@ -87,14 +89,34 @@ constexpr uint64_t kBatchParkLimit = (4ull << 30) / sizeof(grd::Path);
 #endif
 constexpr uint64_t kBatchFills = GR_BATCH_FILLS;
 
-void place_park(Plan &P, Launch &L, int sm_count) {
+// A launch's form and grids.  Small launches take the plain form (plain_tuples), unless they are
+// so deep that a path could be parked: those stay with the pool, which packs their long paths
+// (2,048 tuples of a brilliant at depth 512 2.3 ms, 3.5 with one path per thread and stages).
+void place_blocks(Plan &P, Launch &L, int sm_count) {
     uint64_t tuples = 0;
-    for (uint32_t i = 0; i < L.seg_count; ++i) tuples += P.segs[L.seg_first + i].R.n_tuples;
+    bool shallow = true;  // no path can outlive its segment's drain limit
+    for (uint32_t i = 0; i < L.seg_count; ++i) {
+        const grd::BatchSegment &g = P.segs[L.seg_first + i];
+        tuples += g.R.n_tuples;
+        shallow = shallow && P.slots[g.scene].S.max_bounces / grd::DRAIN_CAPS < g.stage_cap;
+    }
+    P.max_segs = std::max(P.max_segs, L.seg_count);
+    L.blocks = 0;
     const uint64_t T = grh::batch_threads(L.K);
+    const bool clear = L.K >= 0 && (L.K & grd::K_CLEAR);
+    if (shallow && tuples < grd::plain_tuples(L.K < 0)) {
+        L.lanes = grd::plain_lanes(tuples, clear);
+        L.chunk = L.lanes * (grd::TRACE_THREADS / 32);
+        for (uint32_t i = 0; i < L.seg_count; ++i) {
+            grd::BatchSegment &g = P.segs[L.seg_first + i];
+            g.block_begin = L.blocks;
+            L.blocks += (g.R.n_tuples + L.chunk - 1) / L.chunk;
+        }
+        return;
+    }
     uint64_t fills = tuples / ((uint64_t)(sm_count > 0 ? sm_count : 1) * 1024u);
     fills = std::min<uint64_t>(std::max<uint64_t>(fills, 1), kBatchFills);
     L.chunk = (uint32_t)(T * fills);
-    L.blocks = 0;
     const double scale = std::min(1.0 / 16.0, (double)kBatchParkLimit / (double)std::max<uint64_t>(tuples, 1));
     uint64_t off = 0, blocks = 0;
     for (uint32_t i = 0; i < L.seg_count; ++i) {
@@ -112,7 +134,6 @@ void place_park(Plan &P, Launch &L, int sm_count) {
     L.park_paths = off;
     L.park_blocks = blocks;
     P.max_park = std::max(P.max_park, off);
-    P.max_segs = std::max(P.max_segs, L.seg_count);
 }
 
 // Cuts the items into launches of at most `budget` tuples (a pixel whose spp alone
@@ -120,12 +141,12 @@ void place_park(Plan &P, Launch &L, int sm_count) {
 // until the scratch is placed.
 gr_status make_plan(gr_ctx *ctx, const grh::BatchItem *items, uint32_t n_items, uint64_t budget, Plan &P) {
     std::unordered_map<uint64_t, uint32_t> slot_of;
-    const Launch none{0, 0, 0, 0, 0, false, 0, 0, 0, -1};
+    const Launch none{0, 0, 0, 0, 0, false, 0, 0, 0, 0, -1};
     Launch cur = none;
     uint64_t used = 0;
     auto close = [&]() {
         if (cur.seg_count) {
-            place_park(P, cur, ctx->sm_count);
+            place_blocks(P, cur, ctx->sm_count);
             P.launches.push_back(cur);
         }
         P.max_tuples = std::max(P.max_tuples, used);
@@ -225,14 +246,13 @@ gr_status launch_plan(const Plan &P, const grd::SceneSlot *slots, const grd::Bat
     unsigned int *counts = (unsigned int *)park_buf;
     grd::Path *park = (grd::Path *)((char *)park_buf + (((size_t)P.max_segs * sizeof(unsigned int) + 255) & ~(size_t)255));
     for (const Launch &L : P.launches) {
-        const size_t smem = grd::planes_smem_bytes(L.max_planes);
         GR_CUDA(cudaMemsetAsync(counts, 0, (size_t)L.seg_count * sizeof(unsigned int), s));
+        const grd::BatchLaunch G{slots, segs + L.seg_first, L.seg_count, L.lanes, L.chunk, L.max_planes,
+                                 L.blocks, L.park_blocks, park, counts};
         if (L.extras) {
-            grd::launch_batch_grids<true, grd::K_ANY, GR_TRACE_MIN_BLOCKS>(slots, segs + L.seg_first, L.seg_count, L.chunk, park,
-                                                                           counts, L.blocks, L.park_blocks, smem, grd::camera_smem_bytes(L.max_planes), s);
+            grd::launch_batch_grids<true, grd::K_ANY, GR_TRACE_MIN_BLOCKS>(G, s);
         } else {
-            const gr_status st = grh::launch_batch_class(L.K, slots, segs + L.seg_first, L.seg_count, L.chunk, park, counts,
-                                                         L.blocks, L.park_blocks, smem, grd::camera_smem_bytes(L.max_planes), s);
+            const gr_status st = grh::launch_batch_class(L.K, G, s);
             if (st != GR_OK) return st;
         }
         const unsigned T = 256;
@@ -258,6 +278,7 @@ std::vector<uint64_t> graph_key(const Plan &P, const void *tables, const void *x
     }
     for (const Launch &L : P.launches) {
         k.push_back(((uint64_t)L.chunk << 32) ^ L.blocks);
+        k.push_back(L.lanes);
         k.push_back(((uint64_t)L.seg_count << 32) | L.max_planes | ((uint64_t)L.extras << 31) |
                     ((uint64_t)(uint8_t)(L.K + 1) << 20));
     }

@@ -2,7 +2,7 @@
 // environment and film) in one grid.  Included by gr_batch.cu only.
 #pragma once
 
-#include "gr_stage.cuh"
+#include "gr_transport.cuh"
 
 namespace grd {
 
@@ -50,6 +50,34 @@ __device__ __forceinline__ void load_slot(SceneSlot &dst_slot, const SceneSlot *
     const uint32_t *src = reinterpret_cast<const uint32_t *>(src_slot);
     uint32_t *dst = reinterpret_cast<uint32_t *>(&dst_slot);
     for (uint32_t i = threadIdx.x; i < sizeof(SceneSlot) / 4; i += blockDim.x) dst[i] = src[i];
+}
+
+// A batched launch in the plain kernel's form (gr_transport.cuh): `lanes` tuples of one segment
+// per warp, run to their ends.
+template <bool EXTRAS, int K = K_ANY>
+__global__ void __launch_bounds__(TRACE_THREADS, GR_TRACE_MIN_BLOCKS)
+    k_trace_batch_plain(const SceneSlot *__restrict__ slots, const BatchSegment *__restrict__ segs, uint32_t n_segs,
+                        uint32_t lanes) {
+    __shared__ SceneSlot s_slot;
+    __shared__ uint32_t s_seg;
+    extern __shared__ float4 s_planes[];
+    if (threadIdx.x == 0) s_seg = find_segment<0>(segs, n_segs, blockIdx.x);
+    __syncthreads();
+    const BatchSegment &G = segs[s_seg];
+    load_slot(s_slot, slots + G.scene);
+    __syncthreads();
+    const SceneConst &S = s_slot.S;
+    const SceneBuffers &B = s_slot.B;
+    const Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
+    const LaunchRange R = G.R;
+    const uint64_t t = plain_tuple(blockIdx.x - G.block_begin, lanes, R.n_tuples);
+    if (t >= R.n_tuples) return;
+    uint32_t pixel, sample;
+    tuple_coords(R, t, pixel, sample);
+    Path P;
+    path_init<K>(P, S, pixel, sample, (uint32_t)t);
+    NoCounters nc;
+    store_sample(G.xyz, P, trace_path<NoCounters, false, EXTRAS, K>(P, S, B, PL, nc));
 }
 
 // Stage 1 of a batched launch (the pooled scheme of the single-scene kernels): a block runs
@@ -121,13 +149,29 @@ __global__ void __launch_bounds__(pool_threads<EXTRAS, K>(), pool_blocks(MB, poo
         [&](const Path &q) { store_sample(xyz, q, path_finish<1, false, K, EXTRAS>(q, S, B)); });
 }
 
-// One batched launch's two trace grids for scene class K at MB blocks per SM.
+// The trace grids of one batched launch: its segments, scratch and grid sizes (gr_batch.cu).
+// lanes: the plain form with that many tuples per warp; 0: the pooled form's two grids.
+struct BatchLaunch {
+    const SceneSlot *slots;
+    const BatchSegment *segs;
+    uint32_t n_segs, lanes, chunk, max_planes;
+    uint64_t blocks, park_blocks;
+    Path *park;
+    unsigned int *counts;
+};
+
+// They, for scene class K with MB blocks per SM in the pooled form.
 template <bool EXTRAS, int K, int MB>
-void launch_batch_grids(const SceneSlot *slots, const BatchSegment *segs, uint32_t n_segs, uint32_t chunk, Path *park,
-                        unsigned int *counts, uint64_t blocks, uint64_t park_blocks, size_t smem, size_t cam_smem, cudaStream_t s) {
+void launch_batch_grids(const BatchLaunch &L, cudaStream_t s) {
+    const size_t smem = planes_smem_bytes(L.max_planes);
+    if (L.lanes) {
+        k_trace_batch_plain<EXTRAS, K><<<(unsigned)L.blocks, TRACE_THREADS, smem, s>>>(L.slots, L.segs, L.n_segs, L.lanes);
+        return;
+    }
     constexpr int T = pool_threads<EXTRAS, K>();
-    k_trace_batch<EXTRAS, K, MB><<<(unsigned)blocks, T, smem + cam_smem, s>>>(slots, segs, n_segs, chunk, park, counts);
-    k_trace_batch_cont<EXTRAS, K, MB><<<(unsigned)park_blocks, T, smem, s>>>(slots, segs, n_segs, park, counts);
+    k_trace_batch<EXTRAS, K, MB><<<(unsigned)L.blocks, T, smem + camera_smem_bytes(L.max_planes), s>>>(
+        L.slots, L.segs, L.n_segs, L.chunk, L.park, L.counts);
+    k_trace_batch_cont<EXTRAS, K, MB><<<(unsigned)L.park_blocks, T, smem, s>>>(L.slots, L.segs, L.n_segs, L.park, L.counts);
 }
 
 }  // namespace grd

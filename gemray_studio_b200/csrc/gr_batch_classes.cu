@@ -13,15 +13,12 @@
 
 namespace grh {
 
-gr_status launch_batch_class(int K, const grd::SceneSlot *slots, const grd::BatchSegment *segs, uint32_t n_segs,
-                             uint32_t chunk, grd::Path *park, unsigned int *counts, uint64_t blocks, uint64_t park_blocks, size_t smem,
-                             size_t cam_smem, cudaStream_t s) {
+gr_status launch_batch_class(int K, const grd::BatchLaunch &L, cudaStream_t s) {
     constexpr int IC = grd::K_ISO | grd::K_CLEAR;
     constexpr int MB = GR_BATCH_MIN_BLOCKS;
-#define GR_BATCH_CASE(KK)                                                                                       \
-    case KK:                                                                                                    \
-        grd::launch_batch_grids<false, KK, MB>(slots, segs, n_segs, chunk, park, counts, blocks, park_blocks, smem, \
-                                               cam_smem, s);                                                    \
+#define GR_BATCH_CASE(KK)                                  \
+    case KK:                                               \
+        grd::launch_batch_grids<false, KK, MB>(L, s);      \
         break;
     switch (K) {
         GR_BATCH_CASE(IC | grd::k_env(GR_ENV_UNIFORM))

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, GR_TRACE_MIN_BLOCKS)
                          uint32_t lanes) {
     extern __shared__ float4 s_planes[];
     const Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
-    const uint64_t t = plain_tuple(lanes, R.n_tuples);
+    const uint64_t t = plain_tuple(blockIdx.x, lanes, R.n_tuples);
     if (t >= R.n_tuples) return;
     uint32_t pixel, sample;
     tuple_coords(R, t, pixel, sample);
@@ -96,20 +96,12 @@ __global__ void k_stokes_fold(const float4 *__restrict__ iquv, uint32_t n_pixels
 #define GR_STOKES_BLOCKS 12
 #endif
 constexpr int kStokesBlocks = GR_STOKES_BLOCKS;
-// Launches below these sizes run the plain kernel: the pool's 512-thread blocks leave most of
-// the chip idle there and wait at their barriers for the longest scan of the block.  Measured
-// (us of a call, plain / pool): birefringent emerald 16,384 tuples 380 / 553, 131,072 624 /
-// 750, 262,144 878 / 885, 393,216 1523 / 1396; clear brilliant 65,536 472 / 740, 262,144 835 /
-// 1058, 524,288 1670 / 1693; quartz cube 2,048 155 / 258, 131,072 370 / 366; frosted biaxial
-// 16,384 964 / 1337, 65,536 1386 / 1368, 131,072 1970 / 1562.
-constexpr uint64_t kStokesPlain = 1u << 18, kStokesPlainExtras = 1u << 16;
-
 // One launch's samples.  work: the pooled kernel's tuple counter.
 template <bool EXTRAS, int K>
 void launch_stokes(const SceneConst &S, const SceneBuffers &B, const LaunchRange &R, float *xyz, float4 *iquv,
                    unsigned long long *work, uint32_t sm_count, cudaStream_t s) {
     const size_t smem = planes_smem_bytes(S.n_planes);
-    if (R.n_tuples < (EXTRAS ? kStokesPlainExtras : kStokesPlain)) {
+    if (R.n_tuples < plain_tuples(EXTRAS)) {
         const uint32_t lanes = plain_lanes(R.n_tuples, false);
         k_trace_stokes_plain<EXTRAS, K><<<plain_blocks(R.n_tuples, lanes), TRACE_THREADS, smem, s>>>(S, B, R, xyz, iquv, lanes);
         return;

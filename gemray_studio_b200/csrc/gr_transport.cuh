@@ -9,10 +9,11 @@
 
 namespace grd {
 
-// The thread's tuple in a plain launch of `lanes` tuples per warp; `none` for the other lanes.
-__device__ __forceinline__ uint64_t plain_tuple(uint32_t lanes, uint64_t none) {
+// The thread's tuple in block `block` of a plain launch of `lanes` tuples per warp; `none` for
+// the other lanes.
+__device__ __forceinline__ uint64_t plain_tuple(uint64_t block, uint32_t lanes, uint64_t none) {
     const uint32_t lane = threadIdx.x & 31u;
-    return lane < lanes ? ((uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u) * lanes + lane : none;
+    return lane < lanes ? (block * (blockDim.x / 32u) + threadIdx.x / 32u) * lanes + lane : none;
 }
 
 // Plain kernel: one thread traces one tuple start to finish, `lanes` tuples per warp -- the reference
@@ -28,7 +29,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_plain(SceneConst S,
                                                                uint32_t lanes = 32) {
     extern __shared__ float4 s_planes[];
     const Planes PL = stage_scene_planes<EXTRAS, K>(s_planes, S, B);
-    const uint64_t t = plain_tuple(lanes, R.n_tuples);
+    const uint64_t t = plain_tuple(blockIdx.x, lanes, R.n_tuples);
     CT ct;
     if constexpr (sizeof(CT) == sizeof(Counters)) {
         for (int i = 0; i < C_COUNT; ++i) ((Counters &)ct).c[i] = 0;
@@ -71,6 +72,17 @@ inline unsigned plain_blocks(uint64_t n_tuples, uint32_t lanes) {
     const uint64_t per = (uint64_t)lanes * (TRACE_THREADS / 32);
     return (unsigned)((n_tuples + per - 1) / per);
 }
+
+// Batched launches and Stokes films of fewer tuples run in the plain form: the pool's blocks of
+// 256 or 512 threads leave most of the chip idle there and wait at their barriers for the
+// longest scan of the block.  Measured, us of a call, plain / pool.  Batches: quartz cube 2,048
+// tuples 92 / 200, 131,072 394 / 420, 262,144 596 / 544; clear brilliant 16,384 279 / 438,
+// 131,072 454 / 529, 262,144 684 / 636; emerald 131,072 682 / 769, 262,144 967 / 860; frosted
+// biaxial 16,384 852 / 1002, 32,768 977 / 972, 65,536 1285 / 1066.  Stokes films (no scene
+// class): cube 2,048 155 / 258, 131,072 370 / 366; brilliant 65,536 472 / 740, 262,144 835 /
+// 1058; emerald 131,072 624 / 750, 262,144 878 / 885, 393,216 1523 / 1396; frosted biaxial
+// 16,384 964 / 1337, 65,536 1386 / 1368, 131,072 1970 / 1562.
+inline uint64_t plain_tuples(bool extras) { return extras ? 1u << 16 : 1u << 18; }
 
 // Pooled kernels (the scheme and run_pool are in gr_stage.cuh), three launches per trace:
 // k_trace_pool over the launch's tuples, then k_trace_resume over the paths it parked past

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(128) k_guide_pass(SceneConst S, const float4 *
         float d = 1.0e6f;
         V3 n = v3(0.f, 0.f, 0.f);
         int32_t f = -1;
-        int r = intersect_camera(PL, dir, o, t, idx);
+        int r = intersect_camera<true>(PL, dir, o, t, idx);
         if (r == SCAN_UNDECIDED) r = intersect<false>(PL, o, dir, t, idx) ? SCAN_HIT : SCAN_MISS;
         if (r == SCAN_HIT) {
             d = t;

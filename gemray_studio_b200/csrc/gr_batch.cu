@@ -84,10 +84,7 @@ constexpr uint64_t kBatchParkLimit = (4ull << 30) / sizeof(grd::Path);
 // resident threads per SM), at most kBatchFills -- a longer run refills the block's pool more
 // often before it drains, but every SM has to have a block first.  Measured on 64 random
 // stones of 16 to 64 pixels a side (4 / 8 / 16 runs): 28.8 / 28.3 / 29.5 ms.
-#ifndef GR_BATCH_FILLS
-#define GR_BATCH_FILLS 8
-#endif
-constexpr uint64_t kBatchFills = GR_BATCH_FILLS;
+constexpr uint64_t kBatchFills = 8;
 
 // A launch's form and grids.  Small launches take the plain form (plain_tuples), unless they are
 // so deep that a path could be parked: those stay with the pool, which packs their long paths

@@ -9,18 +9,15 @@
 // 64 random stones of 16 to 64 pixels a side, 9 / 12 / 16 blocks: 28.3 / 27.9 / 32.4 ms.  Class
 // K_FULL, whose loops take all channels, at 9 where it is not clear and isotropic (16 absorbing
 // stones of index 1.0002 at 48 x 48 and 32 spp, 9 / 12 blocks: 0.78 / 1.06 ms).
-#ifndef GR_BATCH_MIN_BLOCKS
-#define GR_BATCH_MIN_BLOCKS 12
-#endif
+constexpr int kBatchBlocks = 12;
 
 namespace grh {
 
 gr_status launch_batch_class(int K, const grd::BatchLaunch &L, cudaStream_t s) {
     constexpr int IC = grd::K_ISO | grd::K_CLEAR;
-    constexpr int MB = GR_BATCH_MIN_BLOCKS;
-#define GR_BATCH_CASE(KK)                                  \
-    case KK:                                               \
-        grd::launch_batch_grids<false, KK, MB>(L, s);      \
+#define GR_BATCH_CASE(KK)                                       \
+    case KK:                                                    \
+        grd::launch_batch_grids<false, KK, kBatchBlocks>(L, s); \
         break;
     switch (K) {
         GR_BATCH_CASE(IC | grd::k_env(GR_ENV_UNIFORM))

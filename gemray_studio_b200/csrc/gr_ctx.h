@@ -47,7 +47,7 @@ constexpr uint32_t kScheduleBlocks[kScheduleBlockCount] = {9, 10, 12, 16};
 constexpr uint32_t builtin_schedule_blocks(int scene_class) {
     return scene_class >= 0 && (scene_class & 2 /* grd::K_CLEAR */) ? 16u : 12u;
 }
-// Cap pairs a stone chooses between (of little effect below depths of 64).
+// Cap pairs a stone chooses between (they act from 64 bounces on: DRAIN_CAPS times the least).
 constexpr int kCapPairCount = 3;
 constexpr uint32_t kCapPairs[kCapPairCount][2] = {{12, 20}, {8, 16}, {16, 28}};
 // Candidate schedules: cap pair p at blocks b is candidate p * kScheduleBlockCount + b.

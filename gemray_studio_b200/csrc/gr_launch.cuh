@@ -6,7 +6,8 @@
 //   pixel = first_pixel + t / spp, absolute sample = sample_offset + t % spp,
 // the reference kernel's `idx = pixel * spp + s` numbering
 // (renderer/shaders/spectral_transport.wgsl:672-691), and its XYZ lands in
-// xyz[3 * t .. 3 * t + 3).  The fold then sums each pixel's spp samples in sample
+// xyz[3 * t .. 3 * t + 3), whatever the order in which a launch takes its tuples (pooled
+// launches take a pixel's samples in HeroOrder from 64 on).  The fold then sums each pixel's spp samples in sample
 // order and adds the sum once to the film -- the reference's per-pixel
 // `sum += sample; accum[p] += sum` (renderer/gpu/frame.rs:799-814).
 #pragma once
@@ -125,8 +126,7 @@ __device__ __forceinline__ void store_sample(float *__restrict__ xyz, const Path
 // channels, and a warp runs its channel loops as often as its richest path: 288.8 -> 275.1 ms
 // on the 1080p brilliant at 256 spp, 144.6 -> 140.7 at 128, 4.23 -> 4.16 at 256^2 and 64 spp,
 // 36.9 -> 37.0 at 32 spp, so from 64 samples on; 64 batched stones of 32 to 512 spp 27.5 ->
-// 26.7.  Grouping the classes over several pixels
-// lost more than it gained (38.9 ms at 32 spp).
+// 26.7.  Grouping the classes over several pixels lost more than it gained (38.9 ms at 32 spp).
 constexpr uint32_t HERO_CLASSES = 25, HERO_MIN_SPP = 64;
 struct HeroOrder {
     uint32_t first[HERO_CLASSES + 1];  // samples of one pixel before class k

@@ -1,5 +1,5 @@
 // gr_single.cuh -- launches of the single-scene transport kernels for one scene class K
-// (plain, or the three staged launches over park buffers the caller has prepared).
+// (plain, or the pooled ones over counters and park buffers the caller has prepared).
 // Included by the translation units that instantiate the specialised classes.
 #pragma once
 

@@ -45,11 +45,6 @@ __host__ __device__ constexpr int pool_blocks(int mb, int T) { return mb * 128 /
 #define GR_STAGE_CAP2 20
 #endif
 
-// Unroll factor of the per-channel loops in the pooled kernels' bounce stages.
-#ifndef GR_STEP_UNROLL
-#define GR_STEP_UNROLL 1
-#endif
-
 // Where a draining pool parks the paths past its cap (cap 0: nowhere, they run to their end).
 struct ParkOut {
     Path *park;
@@ -131,10 +126,11 @@ template <int T, uint32_t ROWS> __device__ __forceinline__ void pack_block(Path 
 
 // Runs a block's pool: `start(P, i)` begins item i of the supply in a thread's record,
 // `store(P)` writes a finished path's sample.  Once the supply has run out, paths that have
-// made DRAIN_CAPS * `cap` bounces are parked in `out` while it has slots.  Called by the whole block of
-// T threads; every barrier is reached by all of them.
+// made DRAIN_CAPS * `cap` bounces are parked in `out` while it has slots.  CAM: the planes
+// carry the camera's table.  Called by the whole block of T threads; every barrier is reached
+// by all of them.
 // Packing without a refill (the drain) waits until a quarter of the warps would be freed: a
-// swap costs about a tenth of a bounce.  CAM: the planes carry the camera's table.  Refilling at three quarters instead of half a block
+// swap costs about a tenth of a bounce.  Refilling at three quarters instead of half a block
 // measured 43.3 against 40.5 ms on the brilliant and 48.6 against 43.8 on the emerald: more
 // swaps, and finishes and starts in smaller groups.
 template <int T, bool EXTRAS, int K, bool CAM, class Supply, class Start, class Store>
@@ -196,11 +192,11 @@ __device__ __forceinline__ void run_pool(Path &P, const SceneConst &S, const Sce
         int fidx = 0;
         const bool hit = go && step_scan<NoCounters, false, CAM>(P, PL, t_hit, fidx, nc);
         __syncthreads();
-        if (hit) ev = step_facet<GR_STEP_UNROLL, NoCounters, false, EXTRAS, K>(P, S, B, PL, t_hit, fidx, E, nc);
+        if (hit) ev = step_facet<1, NoCounters, false, EXTRAS, K>(P, S, B, PL, t_hit, fidx, E, nc);
         __syncthreads();
-        if (ev == EV_REFLECT) step_reflect<GR_STEP_UNROLL, NoCounters, EXTRAS, K>(P, S, E, nc);
+        if (ev == EV_REFLECT) step_reflect<1, NoCounters, EXTRAS, K>(P, S, E, nc);
         __syncthreads();
-        if (ev == EV_REFRACT) step_refract<GR_STEP_UNROLL, NoCounters, EXTRAS, K>(P, S, E, nc);
+        if (ev == EV_REFRACT) step_refract<1, NoCounters, EXTRAS, K>(P, S, E, nc);
         if (hit) step_leave(P, PL, fidx);
     }
     if (!(state_bits(P) & F_NONE)) store(P);

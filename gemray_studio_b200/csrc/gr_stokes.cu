@@ -92,10 +92,7 @@ __global__ void k_stokes_fold(const float4 *__restrict__ iquv, uint32_t n_pixels
 
 // Resident blocks per SM of the Stokes kernels, in blocks of 128 threads (384 x 256 emerald at
 // 64 spp: one path per thread 15.8 ms; pooled at 12 / 9 blocks 7.69 / 7.83).
-#ifndef GR_STOKES_BLOCKS
-#define GR_STOKES_BLOCKS 12
-#endif
-constexpr int kStokesBlocks = GR_STOKES_BLOCKS;
+constexpr int kStokesBlocks = 12;
 // One launch's samples.  work: the pooled kernel's tuple counter.
 template <bool EXTRAS, int K>
 void launch_stokes(const SceneConst &S, const SceneBuffers &B, const LaunchRange &R, float *xyz, float4 *iquv,

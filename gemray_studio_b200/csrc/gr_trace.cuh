@@ -210,7 +210,7 @@ __device__ __forceinline__ V3 camera_dir(const SceneConst &S, float x, float y, 
 // Issue-bound like the bounces: with the comb's fmod as a compare and subtract, the lobes'
 // divisions by constants as div_const and the studio lights weighed once per path, the
 // start and end of a path went from 58.2 to 52.3 ms of the 1080p brilliant at 32 spp, 79.2
-// to 70.5 of the 1024^2 emerald at 32 spp (studio), 4.26 to 3.59 of a 317 x 211 tourmaline.
+// to 70.5 of the 1024^2 emerald at 32 spp (studio).
 template <int K = K_ANY>
 __device__ __forceinline__ void path_init(Path &P, const SceneConst &S, uint32_t pixel, uint32_t sample, uint32_t tuple) {
     Draws dr = sample_draws(pixel, sample);
@@ -275,11 +275,12 @@ __device__ __forceinline__ uint32_t channel_tables(Path &P, const SceneConst &S,
 
 // The convex clip (intersect.rs:93-132, simd/slab.rs:101-152).  The reference divides
 // t = -side/denom for every plane, but a plane's t only matters if it can raise the running
-// near maximum (denom < 0) or lower the running far minimum (denom > 0).  q' = (-side) * rcp.approx(denom) is within 2^-21 relative
-// of the exact quotient q; if q' + |q'| 2^-19 < t_near then q < t_near, so the
-// correctly rounded fl(q) <= t_near and the plane cannot update (rounding is
-// monotone) -- likewise for the far side.  Only the remaining planes take the IEEE
-// division, so every t that is compared or kept is the reference's own bits.
+// near maximum (denom < 0) or lower the running far minimum (denom > 0).
+// q' = (-side) * rcp.approx(denom) is within 2^-21 relative of the exact quotient q; if
+// q' + |q'| 2^-19 < t_near then q < t_near, so the correctly rounded fl(q) <= t_near and the
+// plane cannot update (rounding is monotone) -- likewise for the far side.  Only the
+// remaining planes take the IEEE division, so every t that is compared or kept is the
+// reference's own bits.
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -406,7 +407,7 @@ __device__ __forceinline__ bool scan_plane(float denom, float side, int i, float
 // (511 ulp) move v by less than 6.12e-5 of itself, so when the second is not within
 // SCAN_MARGIN of the least, the winner's exact quotient is the strictly least one whatever
 // the rounding.  Only that quotient is then divided, from the same sums as the reference.
-// Facets within the margin (an edge) are settled by their exact quotients .
+// Facets within the margin (an edge) are settled by their exact quotients.
 // Everything else -- a side that is not clearly negative (the origin on or outside a
 // plane, a NaN), no plane to leave through -- returns SCAN_UNDECIDED, and the general scan
 // decides.
@@ -434,15 +435,6 @@ __device__ __forceinline__ float scan_key(float v, uint32_t i) {
     return __uint_as_float((__float_as_uint(v) & ~SCAN_INDEX_MASK) | i);
 }
 
-#ifndef GR_SCAN_UNROLL
-#define GR_SCAN_UNROLL 1
-#endif
-constexpr int SCAN_UNROLL = GR_SCAN_UNROLL;
-#ifndef GR_CAM_UNROLL
-#define GR_CAM_UNROLL 1
-#endif
-constexpr int CAM_UNROLL = GR_CAM_UNROLL;
-
 __device__ __forceinline__ float plane_denom(const float4 &p, V3 d) { return (p.x * d.x + p.y * d.y) + p.z * d.z; }
 __device__ __forceinline__ float plane_side(const float4 &p, V3 o) { return p.w + ((p.x * o.x + p.y * o.y) + p.z * o.z); }
 
@@ -458,7 +450,7 @@ __device__ __forceinline__ int intersect_inside(const Planes &PL, V3 o, V3 d, fl
     const float unit = __uint_as_float(0x3f800000u | (PL.n >> 16));  // 1.0f: n <= GR_MAX_PLANES
     const f32x2 one = pk2(unit, unit);
     float best = 3.0e38f, second = 3.0e38f, side_max = -3.0e38f;
-#pragma unroll SCAN_UNROLL
+#pragma unroll 1
     for (uint32_t i = 0; i < n2; i += 2) {
         const float4 a = PL.pairs[i], b = PL.pairs[i + 1];
         const f32x2 nx = pk2(a.x, a.y), ny = pk2(a.z, a.w), nz = pk2(b.x, b.y);
@@ -539,7 +531,7 @@ __device__ __forceinline__ int intersect_camera(const Planes &PL, V3 d, V3 o, fl
     };
     while (q < q1) {
         const float4 *const some = q + 3 * CAM_PAIRS < q1 ? q + 3 * CAM_PAIRS : q1;
-#pragma unroll CAM_UNROLL
+#pragma unroll 1
         for (; q < some; q += 3) {
             float k0, k1;
             keys(q, k0, k1);
@@ -549,7 +541,7 @@ __device__ __forceinline__ int intersect_camera(const Planes &PL, V3 d, V3 o, fl
         }
         if (near < 0.0f) return SCAN_MISS;  // a plane the origin is beyond, and the ray does not enter
     }
-#pragma unroll CAM_UNROLL
+#pragma unroll 1
     for (; q < q2; q += 3) {
         float k0, k1;
         keys(q, k0, k1);

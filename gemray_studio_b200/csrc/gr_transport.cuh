@@ -1,7 +1,7 @@
 // gr_transport.cuh -- the single-scene transport kernels (sm_100a): the plain kernel
-// (one thread per tuple) and the staged pair (capped first stage, dense continuation),
-// templates over the scene class K (gr_trace.cuh) so that each class is compiled with
-// only the code it runs.  Instantiated by gr_host.cu (the run-time class, counters, FP64
+// (one thread per tuple) and the pooled ones (k_trace_pool, k_trace_resume; the scheme is in
+// gr_stage.cuh), templates over the scene class K (gr_trace.cuh) so that each class is compiled
+// with only the code it runs.  Instantiated by gr_host.cu (the run-time class, counters, FP64
 // re-solve, extension materials) and by gr_single_*.cu (the specialised classes).
 #pragma once
 
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, MB) k_trace_plain(SceneConst S,
 // 643 biaxial; 16,384 tuples 348 / 309 / 295 / 317, 259 / 244 / 257 / 282, 771 / 738 / 751 /
 // 902; 36,864 tuples 405 / 348 / 351 / 412, 263 / 304 / 325 / 445, 780 / 863 / 1023 / 1280.
 inline uint32_t plain_lanes(uint64_t n_tuples, bool clear) {
-    const uint64_t per_lane = 4 * 4 * 148;  // four warps on every scheduler
+    const uint64_t per_lane = 4 * 4 * 148;  // four warps on every scheduler of the B200's 148 SMs
     if (n_tuples <= 4 * per_lane) return 4;
     if (clear) return n_tuples <= 8 * per_lane ? 8 : (n_tuples <= 16 * per_lane ? 16 : 32);
     return n_tuples <= 8 * per_lane ? 16 : 32;

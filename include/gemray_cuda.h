@@ -683,7 +683,7 @@ gr_status gr_denoise_tonemap_device(gr_ctx *ctx, const float *film, uint32_t sam
  * 512 threads (256 for clear isotropic stones) that hold one path per thread, run each
  * bounce together and refill when half of their paths have ended, in three launches: the
  * tuples, then the paths that outlive eight times the schedule's first cap while a block
- * drains, then those past eight times the second (1.85-2.4x the time per sample of the
+ * drains, then those past eight times the second (1.85-2.4x as fast per sample as the
  * earlier one-path-per-thread stages).  AUTO (default): STAGED for launches of at least
  * GR_AUTO_STAGED_MIN_TUPLES tuples; below, PLAIN with 4 to 32 paths per warp, or the first
  * of STAGED's launches alone (scenes with birefringence or absorption from 2^18 tuples,
@@ -714,14 +714,17 @@ gr_status gr_set_kernel(gr_ctx *ctx, uint32_t kernel);
  * caps 8 / 16 and 16 / 28 at the fastest target; the schedule with the least time per
  * tuple is kept for the scene and entered in the context's tuning table.  Writes zeros
  * while the choice is still open (the built-in schedule, caps 12 / 20 at 16 blocks per
- * SM for clear isotropic stones and 12 for others, runs meanwhile).  Batched launches (gr_render_batch, the request loop) run each
- * scene with its chosen first cap, at 12 blocks per SM (their continuation stage is uncapped); gr_accumulate
- * and gr_accumulate_device choose the same way per stone (planes, finishes, material,
- * depth, flags and environment kind; not the view); a frame stream uses its scene's schedule as chosen when
- * the stream opened.  Scenes that need the frosted / scattering / biaxial kernels run
- * those at 9 blocks per SM (two of 512 threads) whatever the schedule's target, scenes with
- * an index outside (1.0005, 8), a gain medium or huge inputs theirs at 12 (clear) or 9.  gr_scene_stage_caps reports
- * the caps alone. */
+ * SM for clear isotropic stones and 12 for others, runs meanwhile).  Two choices launch the
+ * same kernels, and the lesser time of two equal things is kept: 9 and 10 blocks per SM of
+ * stones that are not clear and isotropic (two of 512 threads), and the cap pairs of scenes
+ * of less than 64 bounces.  Batched launches (gr_render_batch, the request loop) run each
+ * scene with its chosen first cap, at 12 blocks per SM (their continuation stage is
+ * uncapped); gr_accumulate and gr_accumulate_device choose the same way per stone (planes,
+ * finishes, material, depth, flags and environment kind; not the view); a frame stream uses
+ * its scene's schedule as chosen when the stream opened.  Scenes that need the frosted /
+ * scattering / biaxial kernels run those at 9 blocks per SM (two of 512 threads) whatever the
+ * schedule's target, scenes with an index outside (1.0005, 8), a gain medium or huge inputs
+ * theirs at 12 (clear) or 9.  gr_scene_stage_caps reports the caps alone. */
 gr_status gr_scene_stage_caps(gr_ctx *ctx, uint64_t scene_id, uint32_t *cap_first, uint32_t *cap_second);
 gr_status gr_scene_schedule(gr_ctx *ctx, uint64_t scene_id, uint32_t *cap_first, uint32_t *cap_second,
                             uint32_t *blocks_per_sm);

@@ -17,8 +17,9 @@ Prints ONE JSON line (rank 0):
   e2e     the same metric through the reference-facing C-ABI call gr_accumulate with
           host buffers (host->device upload of scene + film and the film readback
           inside the timed region);
-  roofline  FP32 bound of the transport (k_trace_pool + k_trace_resume): algorithmic
-          flops from the event-tallied FLOP model / its event-timed duration, against
+  roofline  FP32 bound of the transport (k_trace_pool + k_trace_resume): flops of the
+          reference's arithmetic from the event-tallied FLOP model (all eight channels,
+          of which the kernels skip the ended ones) / its event-timed duration, against
           the FP32 FMA throughput measured on this device;
   cpu_baseline  the C++ restatement of the reference CPU tracer on this host's cores;
   batched / served / accuracy  the metric's other halves, bounded (N=1): C4 at film

@@ -6,9 +6,11 @@ compares, min / max / abs / floor / selects = 0; each transcendental (sin, cos, 
 atan2, acos, libm exp) is one SFU op counted separately, not as flops.  The
 reference's polynomial exp (simd/exp_poly.rs) is ordinary arithmetic: 22 flops.
 
-Per-event costs are static counts of the arithmetic in gemray_studio_b200/csrc
-(gr_device.cuh, gr_trace.cuh), which follows the reference's operation order
-op for op (crates/gemray/src/optics/raytracer/*.rs).
+Per-event costs are static counts of the reference's arithmetic
+(crates/gemray/src/optics/raytracer/*.rs), all eight channels of a path in every event,
+chromatically ended ones included: what the full-sum kernels form, op for op.  The
+default kernels skip ended channels and Mueller terms that are zero, so achieved flops
+over this model say how fast the reference's work is got through; the FP32 units do less.
 """
 from __future__ import annotations
 

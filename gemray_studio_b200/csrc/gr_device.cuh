@@ -72,6 +72,7 @@ struct SceneConst {
     uint32_t has_beta, n_b_bands;
     float b_bands[GR_MAX_BANDS][3];
     uint32_t small_planes;  // every component of every normal within 1e6 (planes_small)
+    uint32_t cam_inside;    // the camera lies inside the stone (Planes::cam_inside)
     uint32_t sane;  // every input finite, no gain, every index in (1.0005, 8) (sane_scene)
 };
 

@@ -367,6 +367,12 @@ void encode_scene(const gr_scene *sc, SceneConst &S) {
     S.map_h = sc->env.latlong_h;
     S.flags = sc->flags;
     S.small_planes = planes_small(sc->planes, sc->n_planes);
+    S.cam_inside = sc->planes && sc->n_planes ? 1u : 0u;
+    for (uint32_t i = 0; S.cam_inside && i < sc->n_planes; ++i) {
+        const gr_plane &p = sc->planes[i];
+        const float side = p.d + (p.normal[0] * S.cam_o[0] + p.normal[1] * S.cam_o[1] + p.normal[2] * S.cam_o[2]);
+        if (!(side < 0.0f)) S.cam_inside = 0u;  // also for NaN
+    }
     S.sane = sane_scene(sc, S) ? 1u : 0u;
 }
 

@@ -46,6 +46,7 @@ template <bool X, int K = K_ANY>
 __device__ __forceinline__ Planes stage_scene_planes(float4 *sp, const SceneConst &S, const SceneBuffers &B) {
     Planes PL = stage_plane_set(sp, B.planes, S.n_planes);
     if (X || (K & K_FULL)) PL.small = S.small_planes != 0;
+    PL.cam_inside = S.cam_inside != 0;
     return PL;
 }
 
